@@ -80,6 +80,8 @@ void free_ws(Workspace &ws) {
   free_dev(ws.orphans);
   free_dev(ws.gpr_scratch);
   free_dev(ws.tc_scratch);
+  free_dev(ws.w64_scratch);
+  ws.w64_bytes = 0;
   ws.tc_scratch_size = 0;
   if (ws.h_flags) cudaFreeHost(ws.h_flags);
   ws.h_flags = nullptr;
@@ -190,7 +192,11 @@ gapgb_status validate_model(gapgb_model *m) {
 
 // Device upload, done by the first call that needs the GPU.
 gapgb_status upload_model(gapgb_model *m) {
-  if (m->d_sf) return GAPGB_OK;
+  if (m->d_sf) {
+    if (m->precision != GAPGB_PREC_FP64 || m->w64_tried) return GAPGB_OK;
+    GAPGB_CUDA_TRY(cudaSetDevice(m->device));
+    return w64_prepare(m);
+  }
   const HostModel &h = m->host;
   int ndev = 0;
   if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev <= 0)
@@ -240,6 +246,10 @@ gapgb_status upload_model(gapgb_model *m) {
   GAPGB_CUDA_TRY(cudaEventCreateWithFlags(&m->ev_join, cudaEventDisableTiming));
   const char *prof = std::getenv("GAPGB_PROFILE_STAGES");
   m->profile_stages = prof && prof[0] && prof[0] != '0';
+  if (m->precision == GAPGB_PREC_FP64) {
+    const gapgb_status st = w64_prepare(m);
+    if (st) return st;
+  }
   m->d_sf = d_sf;  // marks the model as uploaded
   return GAPGB_OK;
 }
@@ -711,6 +721,8 @@ void gapgb_model_free(gapgb_model *m) {
   free_dev(m->d_sf);
   free_dev(m->d_sft64);
   free_dev(m->d_sft32);
+  free_dev(m->d_w64);
+  free_dev(m->d_exp64);
   free_dev(m->d_mmt);
   free_dev(m->d_mmt32);
   free_dev(m->d_invth);
@@ -782,6 +794,11 @@ gapgb_status gapgb_set_option(gapgb_model *m, gapgb_option opt, int64_t value) {
         return fail(GAPGB_ERR_ARG, "attach a surrogate (gapgb_model_set_surrogate) first");
       if (value == GAPGB_PREC_TC && m->host.D > 64)
         return fail(GAPGB_ERR_CAP_EXCEEDED, "tensor-core GPR supports D <= 64");
+      if (value == GAPGB_PREC_FP64 && m->d_sf) {
+        GAPGB_CUDA_TRY(cudaSetDevice(m->device));
+        const gapgb_status st = w64_prepare(m);
+        if (st) return st;
+      }
       m->precision = (int)value;
       return GAPGB_OK;
     case GAPGB_OPT_NEIGHBOUR_CAP:

@@ -215,6 +215,25 @@ inline SFT<T> make_sft(const SFDev &s) {
   return t;
 }
 
+// The FP64 descriptor kernels' table (wacsf64.cu): cutoffs with the scales of
+// the fc polynomial, radial SFs, and the angular SFs grouped by cutoff, each a
+// combination of moments (bern) and of powers of cos (mono), 2^(1-zeta) included.
+constexpr int kFcN = 12;  // coefficients of the fc polynomial
+struct W64Fc {
+  double c[kMaxRC][kFcN];
+};
+struct W64Tab {
+  int nsf, D, nrad, nang, nrc, ngrp, nal, deg;  // nal, deg: the kernels' template sizes
+  double rc[kMaxRC], rc2[kMaxRC], kv[kMaxRC], kd[kMaxRC];
+  int rad_d[kMaxSF], rad_rc[kMaxSF];
+  double rad_alpha[kMaxSF], rad_rs[kMaxSF];
+  int grp_rc[kMaxRC], grp_start[kMaxRC + 1];
+  double alpha[kMaxRC][4];
+  int ang_d[kMaxSF], ang_g[kMaxSF], ang_q[kMaxSF];
+  double bern[kMaxSF][5], mono[kMaxSF][5];
+  W64Fc fc;  // the cutoffs' polynomials (also passed by value, for the constant bank)
+};
+
 struct StructInfo {
   double lat[9];   // rows = lattice vectors
   double linv[9];  // inverse: fractional f = d * linv (row vector)
@@ -292,6 +311,8 @@ struct Workspace {
   size_t gpr_scratch_size = 0;
   void *tc_scratch = nullptr;   // atom operand tiles of the tensor-core GPR
   size_t tc_scratch_size = 0;
+  void *w64_scratch = nullptr;  // wacsf64.cu: moments / scalars of atoms split over blocks
+  size_t w64_bytes = 0;
   // contributing angular pairs (j | k << 8) of every atom, recorded by the
   // grouped FP32 descriptor kernel and streamed by its gradient kernel
   unsigned short *pairs = nullptr;  // [N][kPairCap]
@@ -322,6 +343,10 @@ struct gapgb_model {
   gapgb::SFT<double> *d_sft64 = nullptr;
   gapgb::SFT<float> *d_sft32 = nullptr;
   gapgb::SFT<float> sft32h{};          // host copy (kernel selection)
+  gapgb::W64Tab w64h{};                // FP64 descriptor kernels' table (wacsf64.cu)
+  gapgb::W64Tab *d_w64 = nullptr;
+  double *d_exp64 = nullptr;           // 2^(j/1024)
+  bool w64_tried = false;              // w64_prepare ran (d_w64 stays null: the set does not qualify)
   double *d_mmt = nullptr;             // M x D, mm / theta (FP64)
   float *d_mmt32 = nullptr;            // M x D, mm / theta (FP32)
   double *d_invth = nullptr;           // D, 1 / theta
@@ -423,6 +448,11 @@ void launch_refresh(Workspace &ws, int N, int cap, cudaStream_t st, bool exact =
 template <typename T>
 void launch_wacsf_fwd(const gapgb_model *m, Workspace &ws, int N, int cap, int cap_smem,
                       cudaStream_t st, int a0 = 0, int a1 = -1);
+// wacsf64.cu: the FP64 descriptor kernels of the usual SF sets
+gapgb_status w64_prepare(gapgb_model *m);
+bool w64_applies(const gapgb_model *m, Workspace &ws, int capS, cudaStream_t st);
+void launch_w64_fwd(const gapgb_model *m, Workspace &ws, int N, int cap, int capS, cudaStream_t st);
+void launch_w64_bwd(const gapgb_model *m, Workspace &ws, int N, int cap, int capS, cudaStream_t st);
 // whether the FP32 gradient kernel of this model scatters the forces itself
 // (the reverse slots are then not needed)
 bool bwd_scatters_forces(const gapgb_model *m);

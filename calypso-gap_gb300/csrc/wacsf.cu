@@ -645,6 +645,12 @@ void launch_wacsf_fwd(const gapgb_model *m, Workspace &ws, int N, int cap, int c
       return;
     }
   }
+  if constexpr (std::is_same<T, double>::value) {
+    if (w64_applies(m, ws, capS, st)) {
+      launch_w64_fwd(m, ws, N, cap, capS, st);
+      return;
+    }
+  }
   auto fn = k_wacsf_fwd<T>;
   kernel_smem((const void *)fn, (int)smem);
   int team = 1;
@@ -688,6 +694,12 @@ bool launch_wacsf_bwd(const gapgb_model *m, Workspace &ws, int N, int cap, int c
           (const float *)ws.dedg + (size_t)a0 * D, d_force, ws.wvir + (size_t)a0 * 9,
           ws.pairs + (size_t)a0 * kPairCap, ws.pair_cnt + a0, pcap, ws.d_flags);
       return true;  // forces scattered by the kernel
+    }
+  }
+  if constexpr (std::is_same<T, double>::value) {
+    if (w64_applies(m, ws, capS, st)) {
+      launch_w64_bwd(m, ws, N, cap, capS, st);
+      return false;
     }
   }
   auto fn = k_wacsf_bwd<T>;

@@ -1,0 +1,1036 @@
+// wacsf64.cu - FP64 wACSF descriptors and slot gradients for the usual SF sets
+// (the same functions as wacsf.cu, which holds the reference citations).
+//
+// Taken when every angular SF has an integer zeta of at most 4 and each
+// angular cutoff holds at most 4 distinct alphas; other sets keep wacsf.cu's
+// generic kernels.  GB300 issues FP64 at 1/64 of its FP32 rate (measured 1.06
+// against 78.5 TFLOP/s), so these kernels are bound by the FP64 pipe and are
+// built to issue as few FP64 instructions as possible:
+//  - the pairs of slots within each angular cutoff are found in FP32 from the
+//    neighbour kernel's FP32 records (a conservative screen; the FP64 squared
+//    distance decides) and compacted into lists, so every lane of an FP64
+//    instruction works on a contributing pair;
+//  - fc(r) = (cos(pi r / rc) + 1) / 2 is an even, entire function of r: a
+//    polynomial of degree 11 in r^2, with fc'(r)/r from its derivative, so neither
+//    the slots nor the pairs take a cosine, and a pair takes no square root
+//    and no division either (every factor is written in r^2 and 1/r_slot);
+//  - exp by a 1024-entry table of 2^(j/1024) and a degree-4 polynomial;
+//  - the (1 +- cos)^zeta of a cutoff group are combinations of the products
+//    u^n w^(DEG-n) (u = (1 + cos)/2, w = 1 - u) with non-negative weights: a
+//    pair adds those products, times each alpha's exponential, to moments;
+//  - the gradient contracts dE/dG onto a polynomial in cos per alpha first,
+//    so a pair needs one Horner pass for value and derivative, and it yields
+//    three scalars (s1 + s3, s2 + s3, s3); a slot's gradient is then
+//    d_q sum(s_own + s3) - sum(s3 d_other), gathered per slot.
+// Per pair of the standard set that is about 80 FP64 instructions for the
+// descriptors and 115 for the gradient, where the generic kernels issue about
+// 520 and 770.  Measured (ncu, both generic kernels -> these, split launches
+// included): 512 alloy atoms (56 slots, 690 pairs each) 520 -> 124 us and
+// 665 -> 191 us; 64 carbon atoms (158 slots, 7 cutoffs) 2380 -> 161 us and
+// 1858 -> 329 us.  The FP64 pipe is 62-70 % busy in the larger launches.
+//
+// A block of 4 warps works on one atom.  The pair list of each cutoff group
+// is cut into units of 512 pairs.  Small batches spread an atom's units over
+// several blocks (`split`); the arithmetic is arranged so that the result
+// does not depend on it: moments are summed per unit, units per residue class
+// (unit mod 8) in order, and classes in order; a slot's gradient is summed
+// over its pairs in order after the pairs' scalars are written, by the same
+// block (split = 1) or by a second kernel.  Nothing is atomic, so results are
+// the same bit for bit in every run and in every batch.
+#include <algorithm>
+#include <cmath>
+#include <vector>
+
+#include "gapgb_internal.h"
+
+namespace gapgb {
+namespace {
+
+constexpr int kBlk = 128;        // threads per block (4 warps)
+constexpr int kUnit = 512;       // pairs per unit
+constexpr int kClasses = 8;      // residue classes of units (bounds the split)
+constexpr int kExpN = 1024;      // entries of the 2^(j/1024) table
+
+// fc(r) as a polynomial in v = kv r^2 - 1, -1 <= v <= 1 up to the cutoff
+// (W64Fc::c, formed per cutoff by w64_table), and with its derivative by v.
+// The table is a kernel parameter: its entries are constant-bank operands.
+__device__ __forceinline__ double fc_poly(const double (&c)[kFcN], double v) {
+  double p = c[kFcN - 1];
+#pragma unroll
+  for (int n = kFcN - 2; n >= 0; --n) p = fma(p, v, c[n]);
+  return p;
+}
+__device__ __forceinline__ void fc_poly2(const double (&c)[kFcN], double v, double &p, double &d) {
+  p = fma(c[kFcN - 1], v, c[kFcN - 2]);
+  d = c[kFcN - 1];
+#pragma unroll
+  for (int n = kFcN - 3; n >= 0; --n) {
+    d = fma(d, v, p);
+    p = fma(p, v, c[n]);
+  }
+}
+
+// exp(a b) by table lookup (P. T. P. Tang, "Table-driven implementation of the
+// exponential function in IEEE floating-point arithmetic", ACM TOMS 15, 1989):
+// a b = (1024 n + j) ln2/1024 + r, |r| <= ln2/2048, and e^r - 1 to degree 4
+// (the r^5 term is below 4e-20).  The high part of ln2/1024 has 32 bits, so
+// its multiples are exact and r carries the unrounded product a b.  a1 is
+// a 1024/ln 2.  Outside the normal range, and for NaN, the library's exp.
+constexpr double kPerExp = 1477.3197218702985;  // 1024 / ln 2
+__device__ __forceinline__ double exp_tab(double a, double a1, double b,
+                                          const double *__restrict__ T) {
+  const double kShift = 6755399441055744.0;  // 1.5 2^52: rounds to an integer in the low word
+  const double kf = fma(a1, b, kShift);
+  const int k = __double2loint(kf);
+  const double kd = kf - kShift;
+  if ((__double2hiint(kd) & 0x7fffffff) >= 0x412feb6c) return exp(a * b);  // |a b| >= 708
+  double r = fma(a, b, -(kd * 0x1.62e42fee00000p-11));
+  r = fma(kd, -0x1.a39ef35793c76p-43, r);
+  const double t = T[k & (kExpN - 1)];
+  const double r2 = r * r;
+  double p = fma(r, 1.0 / 24.0, 1.0 / 6.0);
+  p = fma(p, r, 0.5);
+  p = fma(p, r2, r);
+  const double y = fma(t, p, t);
+  return __hiloint2double(__double2hiint(y) + ((k >> 10) << 20), __double2loint(y));
+}
+
+// sums v[0..N) over the warp's lanes by halving exchanges: at each step a
+// lane hands half of its values to its partner and adds the half it keeps
+// (N - 1 additions in all instead of 5 N).  On return *out holds the total of
+// value `idx` (idx < 0: none).  The order of the additions is fixed.
+template <int N>
+__device__ __forceinline__ void warp_fold(double (&v)[N], int lane, double *out, int *idx) {
+  constexpr int P = 32;
+  double a[P];
+#pragma unroll
+  for (int n = 0; n < P; ++n) a[n] = n < N ? v[n] : 0.0;
+  int base = 0;
+#pragma unroll
+  for (int h = 16; h >= 1; h >>= 1) {
+    const bool up = (lane & h) != 0;
+#pragma unroll
+    for (int n = 0; n < h; ++n) {
+      // values n (kept by the lower lanes) and n + h (kept by the upper ones)
+      const bool low_live = n < N, high_live = n + h < N;  // before this step: < min(N, 2h)
+      if (!low_live) continue;
+      if (high_live) {
+        const double give = up ? a[n] : a[n + h];
+        const double got = __shfl_xor_sync(0xffffffffu, give, h);
+        a[n] = (up ? a[n + h] : a[n]) + got;
+      } else {
+        const double got = __shfl_xor_sync(0xffffffffu, a[n], h);
+        a[n] = a[n] + got;  // every lane keeps it; the lower lanes' copy counts
+      }
+    }
+    if (up) base += h;
+  }
+  *out = a[0];
+  *idx = base < N ? base : -1;
+}
+
+// shared-memory layout (bytes), common to the kernels
+struct Lay {
+  size_t A, B, R, fc, f4, idx, mask, pre, row, list, rest, total;
+};
+__host__ __device__ inline size_t up32(size_t x) { return (x + 31) / 32 * 32; }
+__host__ __device__ inline Lay layout(int capS, int nrc, size_t rest) {
+  const int W = (capS + 31) / 32;
+  const size_t c = capS;
+  Lay l;
+  size_t o = kExpN * 8;
+  l.A = o, o += c * 32;                  // dx, dy, dz, r^2/2
+  l.B = o, o += up32(c * 16);            // 1/r, weight
+  l.fc = o, o += up32(c * nrc * 16);     // fc, fc'/r of every cutoff
+  l.f4 = o, o += up32(c * 16);           // FP32 dx, dy, dz, r
+  l.R = o, o += up32(c * 8);             // r
+  l.idx = o, o += up32(c * 2);           // the group's slots (those within its cutoff)
+  l.mask = o, o += up32(c * W * 4);      // pair bits of the group's slots, a row's words adjacent
+  l.pre = o, o += up32(c * W * 2);       // the row's pairs k > j before each word
+  l.row = o, o += up32((c + 2) * 4);     // first pair of each row
+  l.list = o, o += kUnit * 4;            // the unit's pairs
+  l.rest = o, o += up32(rest);
+  l.total = o;
+  return l;
+}
+
+struct View {
+  const double *T;
+  double4 *A;
+  double2 *B, *fc;
+  double *R;
+  float4 *f4;
+  unsigned *mask;
+  unsigned short *idx, *pre;
+  int *row;
+  unsigned *list;
+};
+__device__ __forceinline__ View view(unsigned char *sm, const Lay &l) {
+  View v;
+  v.T = reinterpret_cast<const double *>(sm);
+  v.A = reinterpret_cast<double4 *>(sm + l.A);
+  v.B = reinterpret_cast<double2 *>(sm + l.B);
+  v.fc = reinterpret_cast<double2 *>(sm + l.fc);
+  v.R = reinterpret_cast<double *>(sm + l.R);
+  v.f4 = reinterpret_cast<float4 *>(sm + l.f4);
+  v.idx = reinterpret_cast<unsigned short *>(sm + l.idx);
+  v.mask = reinterpret_cast<unsigned *>(sm + l.mask);
+  v.pre = reinterpret_cast<unsigned short *>(sm + l.pre);
+  v.row = reinterpret_cast<int *>(sm + l.row);
+  v.list = reinterpret_cast<unsigned *>(sm + l.list);
+  return v;
+}
+
+// slots of atom i into shared memory (fc'/r only for the gradient).
+// want_fc: the gather kernel reads positions alone.
+template <bool GRAD>
+__device__ __forceinline__ int stage(const View &s, const W64Tab &t, const W64Fc &fc, int i, int cap, int capS,
+                                     const int *__restrict__ cnt, const double4 *__restrict__ xyzr,
+                                     const int *__restrict__ nj, const double4 *__restrict__ apos,
+                                     const float4 *__restrict__ d32, bool want_fc) {
+  const int P = min(cnt[i], capS);
+  const double4 pi = apos[i];
+  for (int q = threadIdx.x; q < P; q += blockDim.x) {
+    const size_t g = (size_t)i * cap + q;
+    const double4 e = xyzr[g];
+    const double r = e.w;
+    s.A[q] = make_double4(e.x - pi.x, e.y - pi.y, e.z - pi.z, 0.5 * (r * r));
+    s.f4[q] = d32[g];
+    if (!want_fc) continue;
+    s.R[q] = r;
+    s.B[q] = make_double2(1.0 / r, apos[nj[g]].w);
+    for (int c = 0; c < t.nrc; ++c) {
+      double f = 0.0, d = 0.0;
+      if (r <= t.rc[c]) {
+        const double v = fma(r * r, t.kv[c], -1.0);
+        if (GRAD) {
+          fc_poly2(fc.c[c], v, f, d);
+          d *= t.kd[c];
+        } else {
+          f = fc_poly(fc.c[c], v);
+        }
+      }
+      s.fc[(size_t)c * capS + q] = make_double2(f, d);
+    }
+  }
+  return P;
+}
+
+// The pairs j < k of cutoff group g among its n slots (the slots within the
+// cutoff, renumbered in order: idx): bit k of row j's mask words (FULL: for
+// every k, not only k > j), the row's pairs before each word, and the rows'
+// first pairs (row[n] is their number).  FP32 screen with a relative margin
+// of 4e-5 on the squared lengths (the FP32 records are off by less than 1e-6
+// of rc^2): pairs just outside the cutoff may be listed, and contribute
+// exactly zero.  The screen's arithmetic is even in (j, k), so bits (j, k) and
+// (k, j) agree.  Ends with a barrier.
+template <bool FULL>
+__device__ __forceinline__ int build_pairs(const View &s, const W64Tab &t, int g, int P, int &n) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const float rcf = (float)t.rc[t.grp_rc[g]];
+  const float rm = rcf * 1.00002f, c2m = rcf * rcf * 1.00004f;
+  if (warp == 0) {
+    int m = 0;
+    for (int b = 0; b < P; b += 32) {
+      const bool in = b + lane < P && s.f4[b + lane].w <= rm;
+      const unsigned v = __ballot_sync(0xffffffffu, in);
+      if (in) s.idx[m + __popc(v & ((1u << lane) - 1u))] = (unsigned short)(b + lane);
+      m += __popc(v);
+    }
+    if (lane == 0) s.row[P + 1] = m;
+  }
+  __syncthreads();
+  n = s.row[P + 1];
+  const int W = (n + 31) >> 5;
+  for (int j = warp; j < n; j += nw) {
+    const float4 aj = s.f4[s.idx[j]];
+    int c = 0;
+    for (int w = FULL ? 0 : j >> 5; w < W; ++w) {
+      const int k = 32 * w + lane;
+      bool in = k < n && (FULL ? k != j : k > j);
+      const float4 ak = s.f4[s.idx[in ? k : j]];
+      const float cx = aj.x - ak.x, cy = aj.y - ak.y, cz = aj.z - ak.z;
+      in = in && cx * cx + cy * cy + cz * cz <= c2m;
+      const unsigned m = __ballot_sync(0xffffffffu, in);
+      if (lane == 0) {
+        s.mask[j * W + w] = m;
+        s.pre[j * W + w] = (unsigned short)c;
+      }
+      c += __popc(__ballot_sync(0xffffffffu, in && k > j));
+    }
+    if (lane == 0) s.row[j] = c;
+  }
+  __syncthreads();
+  if (warp == 0) {  // exclusive scan of the row counts
+    int carry = 0;
+    for (int b = 0; b < n; b += 32) {
+      const int v = b + lane < n ? s.row[b + lane] : 0;
+      int x = v;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+      }
+      __syncwarp();
+      if (b + lane < n) s.row[b + lane] = carry + x - v;
+      carry += __shfl_sync(0xffffffffu, x, 31);
+    }
+    if (lane == 0) s.row[n] = carry;
+  }
+  __syncthreads();
+  return s.row[n];
+}
+
+// the bits k > j of word w of row j
+__device__ __forceinline__ unsigned upper(const View &s, int W, int j, int w) {
+  const unsigned m = s.mask[j * W + w];
+  return w > (j >> 5) ? m : (w < (j >> 5) ? 0u : m & ~((2u << (j & 31)) - 1u));
+}
+
+// list[p - p0] = j | k << 16 (slots) for the pairs p in [p0, p1).  Ends with a
+// barrier.
+__device__ __forceinline__ void expand(const View &s, int n, int p0, int p1) {
+  const int W = (n + 31) >> 5;
+  for (int j = threadIdx.x; j < n; j += blockDim.x) {
+    int p = s.row[j];
+    if (p >= p1 || s.row[j + 1] <= p0) continue;
+    const unsigned js = s.idx[j];
+    for (int w = j >> 5; w < W && p < p1; ++w) {
+      unsigned m = upper(s, W, j, w);
+      while (m) {
+        const int k = 32 * w + __ffs(m) - 1;
+        m &= m - 1;
+        if (p >= p0 && p < p1) s.list[p - p0] = js | ((unsigned)s.idx[k] << 16);
+        ++p;
+      }
+    }
+  }
+  __syncthreads();
+}
+
+// Descriptors.  grid (atoms, split); block (i, y) takes the units whose
+// residue class is y modulo the split, the last one also the radial terms.
+// split > 1: the classes' moments go to part[i][group][class][moment], summed
+// by k_w64_final.
+template <int NAL, int DEG>
+__global__ void __launch_bounds__(kBlk, NAL * (DEG + 1) <= 10 ? 5 : 3)
+    k_w64_fwd(int N, int cap, int capS, const int *__restrict__ cnt,
+              const double4 *__restrict__ xyzr, const int *__restrict__ nj,
+              const double4 *__restrict__ apos, const float4 *__restrict__ d32,
+              const W64Tab *__restrict__ tab, const __grid_constant__ W64Fc fc,
+              const double *__restrict__ expt,
+              double *__restrict__ G, double *__restrict__ part, int split) {
+  constexpr int NB = DEG + 1, NM = 2 * NAL * NB;
+  extern __shared__ __align__(32) unsigned char smraw[];
+  const W64Tab &t = *tab;
+  const Lay l = layout(capS, t.nrc, 0);
+  const View s = view(smraw, l);
+  double *wpart = reinterpret_cast<double *>(smraw + l.rest);      // [4][NM]
+  double *S = wpart + 4 * NM;                                      // [group][class][NM]
+  double *rp = S + (size_t)t.ngrp * kClasses * NM;                 // [2][kBlk]
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  for (int q = tid; q < kExpN; q += kBlk) reinterpret_cast<double *>(smraw)[q] = expt[q];
+  const int y = blockIdx.y;
+  for (int i = blockIdx.x; i < N; i += gridDim.x) {
+    __syncthreads();
+    const int P = stage<false>(s, t, fc, i, cap, capS, cnt, xyzr, nj, apos, d32, true);
+    for (int q = tid; q < t.ngrp * kClasses * NM; q += kBlk) S[q] = 0.0;
+    __syncthreads();
+    double *Gi = G + (size_t)i * t.D;
+    if (t.nrad > 0 && y == split - 1) {
+      // radial terms: thread = (slot group, SF), so the lanes stay busy for
+      // any number of SFs; the slot groups are summed in order
+      const int ng = kBlk / t.nrad, sr = tid % t.nrad, gr = tid / t.nrad;
+      double acc = 0.0, accw = 0.0;
+      if (gr < ng) {
+        const double al = t.rad_alpha[sr], rs = t.rad_rs[sr];
+        const double2 *f = s.fc + (size_t)t.rad_rc[sr] * capS;
+        for (int q = gr; q < P; q += ng) {
+          const double fq = f[q].x, u = s.R[q] - rs;
+          const double e = exp_tab(-al, -al * kPerExp, u * u, s.T);
+          const double v = __double2hiint(fq) != 0 ? e * fq : 0.0;  // beyond the cutoff: zero
+          acc += v;
+          accw = fma(v, s.B[q].y, accw);
+        }
+      }
+      rp[tid] = acc;
+      rp[kBlk + tid] = accw;
+      __syncthreads();
+      if (tid < t.nrad) {
+        double a = 0.0, w = 0.0;
+        for (int g = 0; g < ng; ++g) {
+          a += rp[g * t.nrad + tid];
+          w += rp[kBlk + g * t.nrad + tid];
+        }
+        Gi[t.rad_d[tid]] = a;
+        Gi[t.rad_d[tid] + t.nsf] = w;
+      }
+    }
+    int u0 = 0;  // index of the group's first unit
+    for (int g = 0; g < t.ngrp; ++g) {
+      __syncthreads();
+      int n;
+      const int np = build_pairs<false>(s, t, g, P, n);
+      const int rci = t.grp_rc[g];
+      const double rc2 = t.rc2[rci], kv = t.kv[rci];
+      const double2 *f = s.fc + (size_t)rci * capS;
+      double al[NAL], al1[NAL];
+#pragma unroll
+      for (int q = 0; q < NAL; ++q) {
+        al[q] = -t.alpha[g][q];
+        al1[q] = al[q] * kPerExp;
+      }
+      const int nu = (np + kUnit - 1) / kUnit;
+      for (int u = 0; u < nu; ++u) {
+        const int cls = (u0 + u) % kClasses;
+        if (cls % split != y) continue;
+        const int p0 = u * kUnit, p1 = min(np, p0 + kUnit);
+        expand(s, n, p0, p1);
+        double acc[NM];
+#pragma unroll
+        for (int n = 0; n < NM; ++n) acc[n] = 0.0;
+        for (int p = p0 + tid; p - lane < p1; p += kBlk) {
+          const bool live = p < p1;
+          const unsigned jk = live ? s.list[p - p0] : 0u;
+          const int j = jk & 0xffff, k = jk >> 16;
+          const double4 aj = s.A[j], ak = s.A[k];
+          const double cx = aj.x - ak.x, cy = aj.y - ak.y, cz = aj.z - ak.z;
+          const double c2 = fma(cx, cx, fma(cy, cy, cz * cz));
+          const double2 bj = s.B[j], bk = s.B[k];
+          double fcc = fc_poly(fc.c[rci], fma(c2, kv, -1.0));
+          const bool in = live && c2 <= rc2;  // else exactly zero
+          fcc = in ? fcc : 0.0;
+          // costheta = (rij^2 + rik^2 - rjk^2) / (2 rij rik) (wacsf.f90:271-273)
+          const double sab = aj.w + ak.w;
+          const double cosv = fma(-0.5, c2, sab) * (bj.x * bk.x);
+          const double s3 = fma(2.0, sab, c2);
+          const double F = f[j].x * f[k].x * fcc;
+          const double wjk = bj.y * bk.y;
+          const double uu = fma(0.5, cosv, 0.5), ww = fma(-0.5, cosv, 0.5);
+          double basis[NB];
+          if constexpr (DEG == 1) {
+            basis[0] = ww;
+            basis[1] = uu;
+          } else if constexpr (DEG == 2) {
+            basis[0] = ww * ww;
+            basis[1] = uu * ww;
+            basis[2] = uu * uu;
+          } else {
+            const double u2 = uu * uu, w2 = ww * ww, uw = uu * ww;
+            basis[0] = w2 * w2;
+            basis[1] = uw * w2;
+            basis[2] = u2 * w2;
+            basis[3] = uw * u2;
+            basis[4] = u2 * u2;
+          }
+#pragma unroll
+          for (int q = 0; q < NAL; ++q) {
+            const double ef = in ? exp_tab(al[q], al1[q], s3, s.T) * F : 0.0;
+            const double efw = ef * wjk;
+#pragma unroll
+            for (int n = 0; n < NB; ++n) {
+              acc[q * NB + n] = fma(basis[n], ef, acc[q * NB + n]);
+              acc[(NAL + q) * NB + n] = fma(basis[n], efw, acc[(NAL + q) * NB + n]);
+            }
+          }
+        }
+        if constexpr (NM <= 32) {
+          double tot;
+          int idx;
+          warp_fold<NM>(acc, lane, &tot, &idx);
+          if (idx >= 0) wpart[warp * NM + idx] = tot;
+        } else {
+          double lo[32], hi[NM - 32], tot;
+          int idx;
+#pragma unroll
+          for (int n = 0; n < NM; ++n) (n < 32 ? lo[n & 31] : hi[n < 32 ? 0 : n - 32]) = acc[n];
+          warp_fold<32>(lo, lane, &tot, &idx);
+          if (idx >= 0) wpart[warp * NM + idx] = tot;
+          warp_fold<NM - 32>(hi, lane, &tot, &idx);
+          if (idx >= 0) wpart[warp * NM + 32 + idx] = tot;
+        }
+        __syncthreads();
+        if (tid < NM)
+          S[(g * kClasses + cls) * NM + tid] +=
+              ((wpart[tid] + wpart[NM + tid]) + wpart[2 * NM + tid]) + wpart[3 * NM + tid];
+      }
+      u0 += nu;
+    }
+    __syncthreads();
+    if (split > 1) {
+      for (int e = tid; e < t.ngrp * kClasses * NM; e += kBlk)
+        if ((e / NM) % kClasses % split == y)
+          part[(size_t)i * t.ngrp * kClasses * NM + e] = S[e];
+    } else {
+      // classes in order, then the moments combine into the SFs
+      for (int e = tid; e < t.ngrp * NM; e += kBlk) {
+        const int g = e / NM, n = e % NM;
+        double v = 0.0;
+        for (int c = 0; c < kClasses; ++c) v += S[(g * kClasses + c) * NM + n];
+        S[(g * kClasses) * NM + n] = v;
+      }
+      __syncthreads();
+      for (int a = tid; a < t.nang; a += kBlk) {
+        const double *m = S + (size_t)t.ang_g[a] * kClasses * NM + t.ang_q[a] * NB;
+        double x = 0.0, w = 0.0;
+#pragma unroll
+        for (int n = 0; n < NB; ++n) {
+          x = fma(t.bern[a][n], m[n], x);
+          w = fma(t.bern[a][n], m[NAL * NB + n], w);
+        }
+        Gi[t.ang_d[a]] = x;
+        Gi[t.ang_d[a] + t.nsf] = w;
+      }
+    }
+  }
+}
+
+// split > 1: the class sums and the combination of moments, as above
+__global__ void __launch_bounds__(kBlk)
+    k_w64_final(int N, int NB, int NM, const W64Tab *__restrict__ tab,
+                const double *__restrict__ part, double *__restrict__ G) {
+  const W64Tab &t = *tab;
+  const int i = blockIdx.x;
+  for (int a = threadIdx.x; a < t.nang; a += kBlk) {
+    const double *m =
+        part + (size_t)i * t.ngrp * kClasses * NM + (size_t)t.ang_g[a] * kClasses * NM + t.ang_q[a] * NB;
+    double x = 0.0, w = 0.0;
+    for (int n = 0; n < NB; ++n) {
+      double mx = 0.0, mw = 0.0;
+      for (int c = 0; c < kClasses; ++c) {
+        mx += m[c * NM + n];
+        mw += m[c * NM + NM / 2 + n];
+      }
+      x = fma(t.bern[a][n], mx, x);
+      w = fma(t.bern[a][n], mw, w);
+    }
+    G[(size_t)i * t.D + t.ang_d[a]] = x;
+    G[(size_t)i * t.D + t.ang_d[a] + t.nsf] = w;
+  }
+}
+
+// adds group g's pairs to the slots' sums: acc[q] = (sum of the neighbour
+// vectors' terms x, y, z; the sum that multiplies d_q).  Two threads per slot,
+// which take the mask words of even and of odd number, each in ascending
+// order; `sc` holds a pair's (s1 + s3, s2 + s3, s3) in one 32-byte sector.
+__device__ __forceinline__ void gather(const View &s, int n, const double4 *sc, double4 *acc) {
+  const int W = (n + 31) >> 5, per = blockDim.x >> 1;
+  for (int q0 = 0; q0 < n; q0 += per) {
+    const int q = q0 + (int)(threadIdx.x >> 1);
+    const bool own = q < n;
+    double4 a = make_double4(0.0, 0.0, 0.0, 0.0);
+    const int wq = q >> 5;
+    const unsigned below = (1u << (q & 31)) - 1u;
+    if (own)
+      for (int w = threadIdx.x & 1; w < W; w += 2) {
+        unsigned m = s.mask[q * W + w];
+        int up = s.row[q] + s.pre[q * W + w];  // the row's next pair (q, k > q)
+        while (m) {
+          const int k = 32 * w + __ffs(m) - 1;
+          m &= m - 1;
+          const bool first = k > q;
+          const int e = first ? up++
+                              : s.row[k] + s.pre[k * W + wq] + __popc(upper(s, W, k, wq) & below);
+          const double *v = reinterpret_cast<const double *>(sc + e);
+          const double4 d = s.A[s.idx[k]];
+          const double c = v[2];
+          a.x = fma(-c, d.x, a.x);
+          a.y = fma(-c, d.y, a.y);
+          a.z = fma(-c, d.z, a.z);
+          a.w += v[first ? 0 : 1];
+        }
+      }
+    a.x += __shfl_xor_sync(0xffffffffu, a.x, 1);
+    a.y += __shfl_xor_sync(0xffffffffu, a.y, 1);
+    a.z += __shfl_xor_sync(0xffffffffu, a.z, 1);
+    a.w += __shfl_xor_sync(0xffffffffu, a.w, 1);
+    if (own && !(threadIdx.x & 1)) {
+      double4 &o = acc[s.idx[q]];
+      o = make_double4(o.x + a.x, o.y + a.y, o.z + a.z, o.w + a.w);
+    }
+  }
+}
+
+// slot gradients and the per-atom virial from the finished sums (the block's
+// first kBlk threads, so that every launch adds in the same order)
+__device__ __forceinline__ void finish(const View &s, int i, int cap, int P, const double4 *acc,
+                                       double *vir, double4 *__restrict__ gslot,
+                                       double *__restrict__ wvir) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (threadIdx.x < kBlk) {
+    double V[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+    for (int q = threadIdx.x; q < P; q += kBlk) {
+      const double4 a = acc[q], d = s.A[q];
+      const double gx = fma(a.w, d.x, a.x), gy = fma(a.w, d.y, a.y), gz = fma(a.w, d.z, a.z);
+      gslot[(size_t)i * cap + q] = make_double4(gx, gy, gz, 0.0);
+      const double dd[3] = {d.x, d.y, d.z}, gg[3] = {gx, gy, gz};
+#pragma unroll
+      for (int x = 0; x < 3; ++x)
+#pragma unroll
+        for (int y = 0; y < 3; ++y) V[x * 3 + y] = fma(dd[x], gg[y], V[x * 3 + y]);
+    }
+    double tot;
+    int idx;
+    warp_fold<9>(V, lane, &tot, &idx);
+    if (idx >= 0) vir[warp * 9 + idx] = tot;
+  }
+  __syncthreads();
+  if (threadIdx.x < 9)
+    wvir[(size_t)i * 9 + threadIdx.x] =
+        ((vir[threadIdx.x] + vir[9 + threadIdx.x]) + vir[18 + threadIdx.x]) + vir[27 + threadIdx.x];
+}
+
+// Slot gradients.  split = 1: grid-stride over atoms; a group's scalars pass
+// through the block's own scratch (sc + blockIdx.x * nsc) and are gathered
+// before the next group.  split > 1: block (i, y) writes its units' scalars
+// to sc + i * nsc + (group's first unit) * kUnit and the radial sums to
+// rad[i][slot], for k_w64_gather.
+template <int NAL, int DEG>
+__global__ void __launch_bounds__(kBlk, 4)
+    k_w64_bwd(int N, int cap, int capS, const int *__restrict__ cnt,
+              const double4 *__restrict__ xyzr, const int *__restrict__ nj,
+              const double4 *__restrict__ apos, const float4 *__restrict__ d32,
+              const W64Tab *__restrict__ tab, const __grid_constant__ W64Fc fc,
+              const double *__restrict__ expt, const double *__restrict__ dedg,
+              double4 *__restrict__ gslot, double *__restrict__ wvir, double4 *scr,
+              double *__restrict__ rad, size_t nsc, int split) {
+  constexpr int NB = DEG + 1;
+  extern __shared__ __align__(32) unsigned char smraw[];
+  const W64Tab &t = *tab;
+  const Lay l = layout(capS, t.nrc, 0);
+  const View s = view(smraw, l);
+  double4 *acc = reinterpret_cast<double4 *>(smraw + l.rest);             // [capS]
+  double *dg = reinterpret_cast<double *>(acc + capS);                    // [D]
+  double *sU = dg + t.D;                                                  // [2][NAL][NB]
+  double *vir = sU + 2 * NAL * NB;                                        // [4][9]
+  const int tid = threadIdx.x, lane = tid & 31;
+  for (int q = tid; q < kExpN; q += kBlk) reinterpret_cast<double *>(smraw)[q] = expt[q];
+  const int y = blockIdx.y;
+  for (int i = blockIdx.x; i < N; i += gridDim.x) {
+    __syncthreads();
+    const int P = stage<true>(s, t, fc, i, cap, capS, cnt, xyzr, nj, apos, d32, true);
+    for (int d = tid; d < t.D; d += kBlk) dg[d] = dedg[(size_t)i * t.D + d];
+    __syncthreads();
+    // radial terms, thread = slot: sum_s dE/dG_s G_s'(r)/r, with
+    // (exp fc)'/r = exp (-2 alpha (1 - rs/r) fc + fc'/r)
+    if (y == split - 1)
+      for (int q = tid; q < P; q += kBlk) {
+        const double r = s.R[q], r2 = 2.0 * s.A[q].w;
+        const double2 b = s.B[q];
+        double sum = 0.0;
+        for (int a = 0; a < t.nrad; ++a) {
+          const double2 f = s.fc[(size_t)t.rad_rc[a] * capS + q];
+          if ((__double2hiint(f.x) | __double2hiint(f.y)) == 0) continue;  // beyond the cutoff
+          const double al = t.rad_alpha[a], rs = t.rad_rs[a];
+          double u2 = r2, ur = 1.0;
+          if (rs != 0.0) {  // uniform over the block
+            const double u = r - rs;
+            u2 = u * u;
+            ur = u * b.x;
+          }
+          const double e = exp_tab(-al, -al * kPerExp, u2, s.T);
+          const double g = fma(-2.0 * al * ur, f.x, f.y);
+          sum = fma(fma(dg[t.rad_d[a] + t.nsf], b.y, dg[t.rad_d[a]]) * e, g, sum);
+        }
+        if (split > 1) rad[(size_t)i * capS + q] = sum;
+        else acc[q] = make_double4(0.0, 0.0, 0.0, sum);
+      }
+    int u0 = 0;
+    for (int g = 0; g < t.ngrp; ++g) {
+      __syncthreads();
+      int n;
+      const int np = build_pairs<true>(s, t, g, P, n);
+      const int rci = t.grp_rc[g];
+      const double rc2 = t.rc2[rci], kv = t.kv[rci], kd = t.kd[rci];
+      const double2 *f = s.fc + (size_t)rci * capS;
+      // dE/dG contracted onto polynomials in cos: cell (weighting, alpha, power)
+      for (int c = tid; c < 2 * NAL * NB; c += kBlk) {
+        const int h = c / (NAL * NB), q = (c / NB) % NAL, m = c % NB;
+        double v = 0.0;
+        for (int a = t.grp_start[g]; a < t.grp_start[g + 1]; ++a)
+          if (t.ang_q[a] == q) v = fma(t.mono[a][m], dg[t.ang_d[a] + (h ? t.nsf : 0)], v);
+        sU[c] = v;
+      }
+      double al[NAL], al1[NAL];
+#pragma unroll
+      for (int q = 0; q < NAL; ++q) {
+        al[q] = -t.alpha[g][q];
+        al1[q] = al[q] * kPerExp;
+      }
+      __syncthreads();
+      double4 *sc = split > 1 ? scr + (size_t)i * nsc + (size_t)u0 * kUnit
+                              : scr + (size_t)blockIdx.x * nsc;
+      const int nu = (np + kUnit - 1) / kUnit;
+      for (int u = 0; u < nu; ++u) {
+        if ((u0 + u) % kClasses % split != y) continue;
+        const int p0 = u * kUnit, p1 = min(np, p0 + kUnit);
+        __syncthreads();  // the previous unit's list has been read
+        expand(s, n, p0, p1);
+        for (int p = p0 + tid; p - lane < p1; p += kBlk) {
+          const bool live = p < p1;
+          const unsigned jk = live ? s.list[p - p0] : 0u;
+          const int j = jk & 0xffff, k = jk >> 16;
+          const double4 aj = s.A[j], ak = s.A[k];
+          const double cx = aj.x - ak.x, cy = aj.y - ak.y, cz = aj.z - ak.z;
+          const double c2 = fma(cx, cx, fma(cy, cy, cz * cz));
+          const double2 bj = s.B[j], bk = s.B[k], fj = f[j], fk = f[k];
+          double fcc, fcd;
+          fc_poly2(fc.c[rci], fma(c2, kv, -1.0), fcc, fcd);
+          fcd *= kd;
+          const bool in = live && c2 <= rc2;
+          fcc = in ? fcc : 0.0;
+          fcd = in ? fcd : 0.0;
+          const double iab = bj.x * bk.x;
+          const double sab = aj.w + ak.w;
+          const double cosv = fma(-0.5, c2, sab) * iab;
+          const double s3 = fma(2.0, sab, c2);
+          const double wjk = bj.y * bk.y;
+          double SP = 0.0, SQ = 0.0, SU = 0.0;
+#pragma unroll
+          for (int q = 0; q < NAL; ++q) {
+            const double e = in ? exp_tab(al[q], al1[q], s3, s.T) : 0.0;
+            const double *U0 = sU + q * NB, *U1 = sU + (NAL + q) * NB;
+            double pv = fma(wjk, U1[DEG], U0[DEG]), pd = 0.0;
+#pragma unroll
+            for (int m = DEG - 1; m >= 0; --m) {
+              pd = m == DEG - 1 ? pv : fma(pd, cosv, pv);
+              pv = fma(pv, cosv, fma(wjk, U1[m], U0[m]));
+            }
+            const double x = e * pv;
+            SQ += x;
+            SU = fma(-2.0 * al[q], x, SU);
+            SP = fma(e, pd, SP);
+          }
+          // d/da of [P(cos) E fc(a) fc(b) fc(c)], over a; likewise b and c:
+          //   dcos/da / a = 1/(ab) - cos/a^2,  dcos/dc / c = -1/(ab)
+          const double fab = fj.x * fk.x;
+          const double F = fab * fcc, Qc = SQ * fcc;
+          const double t1 = fma(SP, fma(-cosv, bj.x * bj.x, iab), -SU);
+          const double t2 = fma(SP, fma(-cosv, bk.x * bk.x, iab), -SU);
+          const double t3 = fma(-SP, iab, -SU);
+          const double c3 = fma(F, t3, SQ * fab * fcd);
+          const double c1 = fma(F, t1, Qc * fk.x * fj.y) + c3;
+          const double cc = fma(F, t2, Qc * fj.x * fk.y) + c3;
+          if (live) sc[p] = make_double4(c1, cc, c3, 0.0);
+        }
+      }
+      u0 += nu;
+      __syncthreads();
+      if (split == 1) gather(s, n, sc, acc);
+    }
+    __syncthreads();
+    if (split == 1) finish(s, i, cap, P, acc, vir, gslot, wvir);
+  }
+}
+
+// split > 1: the gathers of every group in order, as k_w64_bwd does with split 1
+constexpr int kGatherThreads = 512;
+__global__ void __launch_bounds__(kGatherThreads)
+    k_w64_gather(int N, int cap, int capS, const int *__restrict__ cnt,
+                 const double4 *__restrict__ xyzr, const int *__restrict__ nj,
+                 const double4 *__restrict__ apos, const float4 *__restrict__ d32,
+                 const W64Tab *__restrict__ tab, const __grid_constant__ W64Fc fc,
+                 double4 *__restrict__ gslot, double *__restrict__ wvir, const double4 *scr,
+                 const double *__restrict__ rad, size_t nsc) {
+  extern __shared__ __align__(32) unsigned char smraw[];
+  const W64Tab &t = *tab;
+  const Lay l = layout(capS, t.nrc, 0);
+  const View s = view(smraw, l);
+  double4 *acc = reinterpret_cast<double4 *>(smraw + l.rest);
+  double *vir = reinterpret_cast<double *>(acc + capS);
+  const int i = blockIdx.x;
+  const int P = stage<false>(s, t, fc, i, cap, capS, cnt, xyzr, nj, apos, d32, false);
+  for (int q = threadIdx.x; q < P; q += blockDim.x)
+    acc[q] = make_double4(0.0, 0.0, 0.0, rad[(size_t)i * capS + q]);
+  int u0 = 0;
+  for (int g = 0; g < t.ngrp; ++g) {
+    __syncthreads();
+    int n;
+    const int np = build_pairs<true>(s, t, g, P, n);
+    gather(s, n, scr + (size_t)i * nsc + (size_t)u0 * kUnit, acc);
+    u0 += (np + kUnit - 1) / kUnit;
+  }
+  __syncthreads();
+  finish(s, i, cap, P, acc, vir, gslot, wvir);
+}
+
+// unevaluated sums of two doubles (about 106 bits), for the table below
+struct DD {
+  double h, l;
+};
+DD dd_sum(double a, double b) {
+  const double s = a + b, t = s - a;
+  return {s, (a - (s - t)) + (b - t)};
+}
+DD dd_add(DD a, DD b) {
+  DD s = dd_sum(a.h, b.h);
+  return dd_sum(s.h, s.l + a.l + b.l);
+}
+DD dd_mul(DD a, DD b) {
+  const double p = a.h * b.h;
+  return dd_sum(p, std::fma(a.h, b.h, -p) + (a.h * b.l + a.l * b.h));
+}
+DD dd_div(DD a, double b) {
+  const double q = a.h / b;
+  const double r = std::fma(-q, b, a.h) + a.l;
+  return dd_sum(q, r / b);
+}
+
+// fc(r) = (cos(k r) + 1) / 2, k = pi / rc, in powers of v = kv r^2 - 1, with
+// kv = 2 / rc^2 cut to 24 bits (so that kv itself brings no error, and v stays
+// within 1 + 2^-23): the power series of cos(sqrt(t)), t = w (1 + v) with
+// w = k^2 / kv, expanded in v to degree 18 and economised to degree 11 by
+// Chebyshev polynomials.  Coefficients rounded once; the result is within
+// 2e-17 of fc, and its derivative within 5e-17.
+void fc_series(double rc, double *kv, double *c) {
+  const double k = kPiRef / rc;
+  *kv = (double)(float)(2.0 / (rc * rc));
+  constexpr int kDeg = 18, kTerms = 28;
+  const DD w = dd_div(dd_mul({k, 0.0}, {k, 0.0}), *kv);
+  DD a[kDeg + 1] = {};
+  DD u = {0.5, 0.0};  // (-w)^n / (2 (2n)!)
+  double row[kTerms + 1] = {1.0};  // C(n, m)
+  for (int n = 0; n <= kTerms; ++n) {
+    for (int m = 0; m <= std::min(n, kDeg); ++m) a[m] = dd_add(a[m], dd_mul(u, {row[m], 0.0}));
+    u = dd_div(dd_mul(u, {-w.h, -w.l}), (2.0 * n + 1.0) * (2.0 * n + 2.0));
+    for (int m = std::min(n + 1, kTerms); m > 0; --m) row[m] += row[m - 1];
+  }
+  a[0] = dd_add(a[0], {0.5, 0.0});
+  double T[kDeg + 1][kDeg + 1] = {};  // T_n in powers of v (exact integers)
+  T[0][0] = 1.0;
+  T[1][1] = 1.0;
+  for (int n = 2; n <= kDeg; ++n)
+    for (int m = 0; m <= n; ++m) T[n][m] = (m ? 2.0 * T[n - 1][m - 1] : 0.0) - T[n - 2][m];
+  for (int n = kDeg; n >= kFcN; --n) {
+    const DD q = dd_div(a[n], -T[n][n]);
+    for (int m = 0; m < n; ++m) a[m] = dd_add(a[m], dd_mul(q, {T[n][m], 0.0}));
+  }
+  for (int m = 0; m < kFcN; ++m) c[m] = a[m].h;
+}
+
+// C(n, k) for n <= 4
+double binom(int n, int k) {
+  double b = 1.0;
+  for (int q = 1; q <= k; ++q) b = b * (n - q + 1) / q;
+  return b;
+}
+
+using Fwd = decltype(&k_w64_fwd<1, 1>);
+using Bwd = decltype(&k_w64_bwd<1, 1>);
+
+template <int NAL>
+void pick_deg(int deg, Fwd *f, Bwd *b) {
+  if (deg <= 1) { *f = k_w64_fwd<NAL, 1>; *b = k_w64_bwd<NAL, 1>; }
+  else if (deg <= 2) { *f = k_w64_fwd<NAL, 2>; *b = k_w64_bwd<NAL, 2>; }
+  else { *f = k_w64_fwd<NAL, 4>; *b = k_w64_bwd<NAL, 4>; }
+}
+void pick(int nal, int deg, Fwd *f, Bwd *b) {
+  if (nal <= 1) pick_deg<1>(deg, f, b);
+  else if (nal <= 2) pick_deg<2>(deg, f, b);
+  else pick_deg<4>(deg, f, b);
+}
+
+int nal_pad(int n) { return n <= 1 ? 1 : (n <= 2 ? 2 : 4); }
+int deg_pad(int d) { return d <= 1 ? 1 : (d <= 2 ? 2 : 4); }
+
+constexpr size_t kSmemMax = 227 * 1024;
+
+// blocks per atom: enough that every SM has about 8 blocks, at most the number
+// of classes (one block per atom from 8 atoms per SM)
+int split_of(int N) {
+  const int want = 8 * device_sms();
+  int s = 1;
+  while (s < kClasses && N * s < want) s *= 2;
+  return s;
+}
+
+}  // namespace
+
+namespace {
+
+// The table of a model, or false when its SF set keeps the generic kernels.
+bool w64_table(const SFDev &s, W64Tab *t) {
+  *t = W64Tab{};
+  t->nsf = s.nsf;
+  t->D = s.D;
+  t->nrad = s.nrad;
+  t->nang = s.nang;
+  t->nrc = s.nrc;
+  t->ngrp = s.n_ang_grp;
+  for (int q = 0; q < s.nrc; ++q) {
+    t->rc[q] = s.rc_val[q];
+    t->rc2[q] = s.rc_val[q] * s.rc_val[q];
+    fc_series(s.rc_val[q], &t->kv[q], t->fc.c[q]);
+    t->kd[q] = 2.0 * t->kv[q];  // fc'(r) / r = (d fc / dv) 2 kv
+  }
+  for (int q = 0; q < s.nrad; ++q) {
+    t->rad_d[q] = s.rad_d[q];
+    t->rad_rc[q] = s.rad_rc[q];
+    t->rad_alpha[q] = s.rad_alpha[q];
+    t->rad_rs[q] = s.rad_rs[q];
+  }
+  int nal = 1, deg = 1;
+  for (int g = 0; g < s.n_ang_grp; ++g) {
+    t->grp_rc[g] = s.ang_grp_rc[g];
+    t->grp_start[g] = s.ang_grp_start[g];
+    t->grp_start[g + 1] = s.ang_grp_start[g + 1];
+    int n = 0;
+    for (int a = s.ang_grp_start[g]; a < s.ang_grp_start[g + 1]; ++a) {
+      if (s.ang_izeta[a] < 1 || s.ang_izeta[a] > 4) return false;
+      deg = deg > s.ang_izeta[a] ? deg : s.ang_izeta[a];
+      const double al = s.alpha_val[s.ang_alpha[a]];
+      int q = 0;
+      while (q < n && t->alpha[g][q] != al) ++q;
+      if (q == 4) return false;
+      if (q == n) t->alpha[g][n++] = al;
+      t->ang_d[a] = s.ang_d[a];
+      t->ang_g[a] = g;
+      t->ang_q[a] = q;
+    }
+    nal = nal > n ? nal : n;
+  }
+  t->nal = nal_pad(nal);
+  t->deg = deg_pad(deg);
+  for (int a = 0; a < s.nang; ++a) {
+    const int z = s.ang_izeta[a], R = t->deg - z;
+    const bool neg = s.ang_lambda[a] < 0;
+    for (int n = 0; n <= t->deg; ++n) {
+      // (1 +- cos)^z = (2u)^z or (2w)^z, times (u + w)^R
+      const int m = neg ? t->deg - n : n;
+      t->bern[a][n] = m >= z ? s.ang_pref[a] * std::ldexp(binom(R, m - z), z) : 0.0;
+      t->mono[a][n] = n <= z ? s.ang_pref[a] * binom(z, n) * ((neg && (n & 1)) ? -1.0 : 1.0) : 0.0;
+    }
+  }
+  return true;
+}
+
+}  // namespace
+
+// The model's table and 2^(j/1024) on the device; called when a model that
+// is on the device takes, or is switched to, the FP64 form.
+gapgb_status w64_prepare(gapgb_model *m) {
+  if (m->d_w64 || m->w64_tried) return GAPGB_OK;
+  m->w64_tried = true;
+  if (!w64_table(m->sfh, &m->w64h)) return GAPGB_OK;
+  static const std::vector<double> T = [] {
+    std::vector<double> v(kExpN);
+    for (int j = 0; j < kExpN; ++j) v[j] = std::exp2((double)j / kExpN);
+    return v;
+  }();
+  GAPGB_CUDA_TRY(cudaMalloc(&m->d_exp64, sizeof(double) * kExpN));
+  GAPGB_CUDA_TRY(cudaMemcpy(m->d_exp64, T.data(), sizeof(double) * kExpN, cudaMemcpyHostToDevice));
+  GAPGB_CUDA_TRY(cudaMalloc(&m->d_w64, sizeof(W64Tab)));
+  GAPGB_CUDA_TRY(cudaMemcpy(m->d_w64, &m->w64h, sizeof(W64Tab), cudaMemcpyHostToDevice));
+  return GAPGB_OK;
+}
+
+namespace {
+
+size_t fwd_smem(const gapgb_model *m, int capS) {
+  const W64Tab &t = m->w64h;
+  const size_t nm = 2 * t.nal * (t.deg + 1);
+  return layout(capS, t.nrc, 8 * (4 * nm + (size_t)t.ngrp * kClasses * nm + 2 * kBlk)).total;
+}
+size_t bwd_smem(const gapgb_model *m, int capS) {
+  const W64Tab &t = m->w64h;
+  return layout(capS, t.nrc,
+                (size_t)capS * 32 + 8 * ((size_t)t.D + 2 * t.nal * (t.deg + 1) + 36))
+      .total;
+}
+// units of one group at most, and scalar records of a block's scratch
+size_t group_units(int capS) {
+  const size_t pairs = (size_t)capS * (capS - 1) / 2;
+  return std::max<size_t>(1, (pairs + kUnit - 1) / kUnit);
+}
+
+// The kernels' scratch, grown as needed.  False when it cannot be had: an
+// allocation failed, the buffer would move while a captured graph holds its
+// address, or the stream is being captured (no allocation there).
+constexpr size_t kScratchMax = (size_t)1 << 30;
+bool scratch(const gapgb_model *m, Workspace &ws, size_t bytes, cudaStream_t st) {
+  if (bytes <= ws.w64_bytes) return true;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (m->live_graphs->load() > 0 || cudaStreamIsCapturing(st, &cap) != cudaSuccess ||
+      cap != cudaStreamCaptureStatusNone)
+    return false;
+  const size_t had = ws.w64_bytes;
+  if (ws.w64_scratch) cudaFree(ws.w64_scratch);
+  for (const size_t b : {bytes, had}) {  // the old size again when the new one fails
+    ws.w64_scratch = nullptr;
+    ws.w64_bytes = 0;
+    if (b > 0 && cudaMalloc(&ws.w64_scratch, b) == cudaSuccess) {
+      ws.w64_bytes = b;
+      break;
+    }
+    cudaGetLastError();
+  }
+  return ws.w64_bytes >= bytes;
+}
+
+}  // namespace
+
+// Whether the kernels take a batch with capS slots per atom.  Also sizes the
+// scratch of the gradient's launch with one block per atom (a region per
+// resident block, fewer blocks when a region is large), so that the gradient
+// of a batch always takes the kernels that its descriptors took.
+bool w64_applies(const gapgb_model *m, Workspace &ws, int capS, cudaStream_t st) {
+  return m->d_w64 && capS < 65536 && fwd_smem(m, capS) <= kSmemMax &&
+         bwd_smem(m, capS) <= kSmemMax && scratch(m, ws, group_units(capS) * kUnit * 32, st);
+}
+
+void launch_w64_fwd(const gapgb_model *m, Workspace &ws, int N, int cap, int capS, cudaStream_t st) {
+  const W64Tab &t = m->w64h;
+  const int NB = t.deg + 1, NM = 2 * t.nal * NB;
+  Fwd f;
+  Bwd b;
+  pick(t.nal, t.deg, &f, &b);
+  const size_t smem = fwd_smem(m, capS);
+  kernel_smem((const void *)f, (int)smem, true);
+  const size_t need = sizeof(double) * (size_t)N * t.ngrp * kClasses * NM;
+  int split = split_of(N);
+  if (split > 1 && (need > kScratchMax || !scratch(m, ws, need, st))) split = 1;
+  const int gx = std::min(N, 1 << 20);
+  f<<<dim3(gx, split), kBlk, smem, st>>>(N, cap, capS, ws.nbr_cnt, ws.nbr_xyz, ws.nbr_j, ws.apos,
+                                         ws.nbr_d32, m->d_w64, m->w64h.fc, m->d_exp64,
+                                         (double *)ws.G, (double *)ws.w64_scratch, split);
+  if (split > 1 && t.nang > 0)
+    k_w64_final<<<N, kBlk, 0, st>>>(N, NB, NM, m->d_w64, (const double *)ws.w64_scratch,
+                                    (double *)ws.G);
+}
+
+void launch_w64_bwd(const gapgb_model *m, Workspace &ws, int N, int cap, int capS, cudaStream_t st) {
+  const W64Tab &t = m->w64h;
+  Fwd f;
+  Bwd b;
+  pick(t.nal, t.deg, &f, &b);
+  const size_t smem = bwd_smem(m, capS);
+  kernel_smem((const void *)b, (int)smem, true);
+  int split = split_of(N);
+  size_t nsc = group_units(capS) * kUnit * std::max(1, t.ngrp), need = 0;
+  if (split > 1) {
+    need = (size_t)N * (nsc * 32 + (size_t)capS * 8);
+    if (need > kScratchMax || !scratch(m, ws, need, st)) split = 1;
+  }
+  int gx = N;
+  if (split == 1) {
+    nsc = group_units(capS) * kUnit;
+    gx = std::min(N, device_sms() * kernel_occupancy((const void *)b, kBlk, smem));
+    gx = (int)std::min<size_t>(gx, std::max<size_t>(1, kScratchMax / (nsc * 32)));
+    if (!scratch(m, ws, gx * nsc * 32, st)) gx = (int)(ws.w64_bytes / (nsc * 32));  // >= 1: w64_applies
+  }
+  double4 *sc = (double4 *)ws.w64_scratch;
+  double *rad = (double *)(sc + (split > 1 ? (size_t)N * nsc : 0));
+  b<<<dim3(gx, split), kBlk, smem, st>>>(N, cap, capS, ws.nbr_cnt, ws.nbr_xyz, ws.nbr_j, ws.apos,
+                                         ws.nbr_d32, m->d_w64, m->w64h.fc, m->d_exp64,
+                                         (const double *)ws.dedg, (double4 *)ws.gslot, ws.wvir, sc,
+                                         rad, nsc, split);
+  if (split > 1) {
+    const size_t sg = layout(capS, t.nrc, (size_t)capS * 32 + 36 * 8).total;
+    kernel_smem((const void *)k_w64_gather, (int)sg, true);
+    k_w64_gather<<<N, kGatherThreads, sg, st>>>(N, cap, capS, ws.nbr_cnt, ws.nbr_xyz, ws.nbr_j,
+                                                ws.apos, ws.nbr_d32, m->d_w64, m->w64h.fc,
+                                                (double4 *)ws.gslot, ws.wvir, sc, rad, nsc);
+  }
+}
+
+}  // namespace gapgb
