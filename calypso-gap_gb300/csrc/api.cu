@@ -28,6 +28,26 @@ static thread_local std::string g_last_error;
 
 void set_last_error(const std::string &s) { g_last_error = s; }
 
+bool grow_scratch(const gapgb_model *m, void **p, size_t *have, size_t bytes, cudaStream_t st) {
+  if (bytes <= *have) return true;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (m->live_graphs->load() > 0 || cudaStreamIsCapturing(st, &cap) != cudaSuccess ||
+      cap != cudaStreamCaptureStatusNone)
+    return false;
+  const size_t had = *have;
+  if (*p) cudaFree(*p);
+  for (const size_t b : {bytes, had}) {  // the old size again when the new one fails
+    *p = nullptr;
+    *have = 0;
+    if (b > 0 && cudaMalloc(p, b) == cudaSuccess) {
+      *have = b;
+      break;
+    }
+    cudaGetLastError();
+  }
+  return *have >= bytes;
+}
+
 namespace {
 
 gapgb_status fail(gapgb_status st, const std::string &msg) {
@@ -82,6 +102,8 @@ void free_ws(Workspace &ws) {
   free_dev(ws.tc_scratch);
   free_dev(ws.w64_scratch);
   ws.w64_bytes = 0;
+  free_dev(ws.g64_scratch);
+  ws.g64_bytes = 0;
   ws.tc_scratch_size = 0;
   if (ws.h_flags) cudaFreeHost(ws.h_flags);
   ws.h_flags = nullptr;
@@ -190,13 +212,23 @@ gapgb_status validate_model(gapgb_model *m) {
   return GAPGB_OK;
 }
 
+// What a precision form keeps on the device beside the model's arrays (the
+// FP64 descriptor tables, the FP64 GPR's digit images), made once.
+gapgb_status prepare_form(gapgb_model *m, int precision) {
+  const bool fp64 = precision == GAPGB_PREC_FP64;
+  const bool gpr64 = fp64 || precision == GAPGB_PREC_MIXED;
+  if ((!fp64 || m->w64_tried) && (!gpr64 || m->g64_tried)) return GAPGB_OK;
+  GAPGB_CUDA_TRY(cudaSetDevice(m->device));
+  if (fp64) {
+    const gapgb_status st = w64_prepare(m);
+    if (st) return st;
+  }
+  return gpr64 ? g64_prepare(m) : GAPGB_OK;
+}
+
 // Device upload, done by the first call that needs the GPU.
 gapgb_status upload_model(gapgb_model *m) {
-  if (m->d_sf) {
-    if (m->precision != GAPGB_PREC_FP64 || m->w64_tried) return GAPGB_OK;
-    GAPGB_CUDA_TRY(cudaSetDevice(m->device));
-    return w64_prepare(m);
-  }
+  if (m->d_sf) return prepare_form(m, m->precision);
   const HostModel &h = m->host;
   int ndev = 0;
   if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev <= 0)
@@ -246,12 +278,8 @@ gapgb_status upload_model(gapgb_model *m) {
   GAPGB_CUDA_TRY(cudaEventCreateWithFlags(&m->ev_join, cudaEventDisableTiming));
   const char *prof = std::getenv("GAPGB_PROFILE_STAGES");
   m->profile_stages = prof && prof[0] && prof[0] != '0';
-  if (m->precision == GAPGB_PREC_FP64) {
-    const gapgb_status st = w64_prepare(m);
-    if (st) return st;
-  }
   m->d_sf = d_sf;  // marks the model as uploaded
-  return GAPGB_OK;
+  return prepare_form(m, m->precision);
 }
 
 int max_struct_atoms(int S, const int *atom_off) {
@@ -415,8 +443,12 @@ gapgb_status enqueue_tail(gapgb_model *m, int S, int N, int cap, int capS, int l
     if (s) return s;
     launch_gpr_tf32(m, ws, N, st);
   }
-  else if (fp64) launch_gpr<double, double>(m, ws, N, st);
-  else if (m->precision == GAPGB_PREC_MIXED) launch_gpr<double, float>(m, ws, N, st);
+  else if (fp64) {
+    if (!launch_gpr64<double>(m, ws, N, st)) launch_gpr<double, double>(m, ws, N, st);
+  }
+  else if (m->precision == GAPGB_PREC_MIXED) {
+    if (!launch_gpr64<float>(m, ws, N, st)) launch_gpr<double, float>(m, ws, N, st);
+  }
   else launch_gpr<float, float>(m, ws, N, st);
   if (prof) cudaEventRecord(m->ev[3], st);
   if (lgrad) {
@@ -723,6 +755,7 @@ void gapgb_model_free(gapgb_model *m) {
   free_dev(m->d_sft32);
   free_dev(m->d_w64);
   free_dev(m->d_exp64);
+  free_dev(m->d_g64);
   free_dev(m->d_mmt);
   free_dev(m->d_mmt32);
   free_dev(m->d_invth);
@@ -794,9 +827,8 @@ gapgb_status gapgb_set_option(gapgb_model *m, gapgb_option opt, int64_t value) {
         return fail(GAPGB_ERR_ARG, "attach a surrogate (gapgb_model_set_surrogate) first");
       if (value == GAPGB_PREC_TC && m->host.D > 64)
         return fail(GAPGB_ERR_CAP_EXCEEDED, "tensor-core GPR supports D <= 64");
-      if (value == GAPGB_PREC_FP64 && m->d_sf) {
-        GAPGB_CUDA_TRY(cudaSetDevice(m->device));
-        const gapgb_status st = w64_prepare(m);
+      if (m->d_sf) {
+        const gapgb_status st = prepare_form(m, (int)value);
         if (st) return st;
       }
       m->precision = (int)value;
@@ -878,7 +910,7 @@ gapgb_status gapgb_model_set_coeff(gapgb_model *m, const double *coeff) {
     const gapgb_status st = build_tf32_image(m, true);
     if (st) return st;
   }
-  return GAPGB_OK;
+  return g64_prepare(m, true);
 }
 
 gapgb_status gapgb_fit(gapgb_model *m, int nstruct, const int *atom_off, const int *species,

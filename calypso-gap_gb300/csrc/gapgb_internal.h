@@ -313,6 +313,8 @@ struct Workspace {
   size_t tc_scratch_size = 0;
   void *w64_scratch = nullptr;  // wacsf64.cu: moments / scalars of atoms split over blocks
   size_t w64_bytes = 0;
+  void *g64_scratch = nullptr;  // gpr64_tc.cu: operands, kernel values, partial sums
+  size_t g64_bytes = 0;
   // contributing angular pairs (j | k << 8) of every atom, recorded by the
   // grouped FP32 descriptor kernel and streamed by its gradient kernel
   unsigned short *pairs = nullptr;  // [N][kPairCap]
@@ -359,6 +361,8 @@ struct gapgb_model {
   void *d_tf32 = nullptr;              // TF32 operand images (gpr_tf32.cu)
   size_t tf32_bytes = 0;
   int tf32_tiles = 0;
+  unsigned char *d_g64 = nullptr;      // digit images of the FP64 tensor-core GPR (gpr64_tc.cu)
+  bool g64_tried = false;              // g64_prepare ran (d_g64 stays null: the model does not qualify)
   int device = 0;
   int precision = GAPGB_PREC_FP64;
   int cap = 256;
@@ -448,6 +452,14 @@ void launch_refresh(Workspace &ws, int N, int cap, cudaStream_t st, bool exact =
 template <typename T>
 void launch_wacsf_fwd(const gapgb_model *m, Workspace &ws, int N, int cap, int cap_smem,
                       cudaStream_t st, int a0 = 0, int a1 = -1);
+// A kernel's scratch in the workspace, grown as needed.  False when it cannot
+// be had: an allocation failed, the buffer would move while a captured graph
+// holds its address, or the stream is being captured (no allocation there).
+bool grow_scratch(const gapgb_model *m, void **p, size_t *have, size_t bytes, cudaStream_t st);
+// gpr64_tc.cu: the FP64 GPR on the tensor cores
+gapgb_status g64_prepare(gapgb_model *m, bool refresh = false);
+template <typename TG>
+bool launch_gpr64(const gapgb_model *m, Workspace &ws, int N, cudaStream_t st);
 // wacsf64.cu: the FP64 descriptor kernels of the usual SF sets
 gapgb_status w64_prepare(gapgb_model *m);
 bool w64_applies(const gapgb_model *m, Workspace &ws, int capS, cudaStream_t st);

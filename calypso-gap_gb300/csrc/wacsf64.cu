@@ -943,28 +943,9 @@ size_t group_units(int capS) {
   return std::max<size_t>(1, (pairs + kUnit - 1) / kUnit);
 }
 
-// The kernels' scratch, grown as needed.  False when it cannot be had: an
-// allocation failed, the buffer would move while a captured graph holds its
-// address, or the stream is being captured (no allocation there).
 constexpr size_t kScratchMax = (size_t)1 << 30;
 bool scratch(const gapgb_model *m, Workspace &ws, size_t bytes, cudaStream_t st) {
-  if (bytes <= ws.w64_bytes) return true;
-  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  if (m->live_graphs->load() > 0 || cudaStreamIsCapturing(st, &cap) != cudaSuccess ||
-      cap != cudaStreamCaptureStatusNone)
-    return false;
-  const size_t had = ws.w64_bytes;
-  if (ws.w64_scratch) cudaFree(ws.w64_scratch);
-  for (const size_t b : {bytes, had}) {  // the old size again when the new one fails
-    ws.w64_scratch = nullptr;
-    ws.w64_bytes = 0;
-    if (b > 0 && cudaMalloc(&ws.w64_scratch, b) == cudaSuccess) {
-      ws.w64_bytes = b;
-      break;
-    }
-    cudaGetLastError();
-  }
-  return ws.w64_bytes >= bytes;
+  return grow_scratch(m, &ws.w64_scratch, &ws.w64_bytes, bytes, st);
 }
 
 }  // namespace
