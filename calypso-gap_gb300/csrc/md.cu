@@ -244,7 +244,7 @@ gapgb_status gapgb_md_create(gapgb_model *m, int nstruct, int natoms, const int 
   md->d_pos = d_pos;
   md->d_vel = d_vel;
   md->d_mass = d_mass;
-  md->kin_parts = std::max(1, std::min(kKinParts, natoms / nstruct / 2048));
+  md->kin_parts = std::max(1, std::min(kKinParts, natoms / nstruct / 512));
   gapgb_status st = md_prepare(m, natoms, nstruct);
   if (st) {
     gapgb_md_free(md);

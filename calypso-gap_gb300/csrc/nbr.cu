@@ -28,98 +28,124 @@ __device__ __forceinline__ void crossp_rn(const double *a, const double *b, doub
   o[2] = __dsub_rn(__dmul_rn(a[0], b[1]), __dmul_rn(a[1], b[0]));
 }
 
-// One thread per structure: image counts (gap_calc.f90:85-88 with
+// 16 lanes per structure: image counts (gap_calc.f90:85-88 with
 // recipvector/volume/crossp of :240-266, same operation order), volume
-// (det, :201 and :290-299) and the inverse lattice for pruning.
-__global__ void k_prep_struct(int S, const int *__restrict__ atom_off,
-                              const double *__restrict__ lat_all, double rcut, int allow_bins,
-                              StructInfo *__restrict__ out, int *__restrict__ flags) {
-  int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= S) return;
-  StructInfo si;
-  const double *L = lat_all + (size_t)s * 9;
-  for (int q = 0; q < 9; ++q) si.lat[q] = L[q];
+// (det, :201 and :290-299) and the inverse lattice for pruning.  The chain of
+// FP64 divisions and roots is what this kernel takes; a lane per reciprocal
+// component and per inverse entry shortens it from 18 divisions in a row to 4
+// (23 -> 9 us, a tenth of a 64-atom call).
+constexpr int kPrepLanes = 16;
+__global__ void __launch_bounds__(128)
+    k_prep_struct(int S, const int *__restrict__ atom_off, const double *__restrict__ lat_all,
+                  double rcut, int allow_bins, StructInfo *__restrict__ out,
+                  int *__restrict__ flags) {
+  const int q = threadIdx.x % kPrepLanes, base = threadIdx.x & 16;
+  int s = (blockIdx.x * blockDim.x + threadIdx.x) / kPrepLanes;
+  const bool live = s < S;
+  s = live ? s : S - 1;  // idle lanes repeat the last structure (shuffles stay full)
+  double L[9];
+#pragma unroll
+  for (int t = 0; t < 9; ++t) L[t] = lat_all[(size_t)s * 9 + t];
   // Fortran LAT(i,j) = L[(i-1)*3 + (j-1)]; columns c_j = LAT(:,j)
-  double c1[3] = {L[0], L[3], L[6]}, c2[3] = {L[1], L[4], L[7]}, c3[3] = {L[2], L[5], L[8]};
-  double r1[3], r2[3], r3[3];
-  crossp_rn(c2, c3, r1);
-  crossp_rn(c3, c1, r2);
-  crossp_rn(c1, c2, r3);
-  double vol = fabs(__dadd_rn(__dadd_rn(__dmul_rn(c1[0], r1[0]), __dmul_rn(c1[1], r1[1])),
-                              __dmul_rn(c1[2], r1[2])));
-  double *cols[3] = {r1, r2, r3};
-  for (int a = 0; a < 3; ++a)
-    for (int b = 0; b < 3; ++b)
-      cols[a][b] = __dmul_rn(__dmul_rn(__ddiv_rn(cols[a][b], vol), kPiRef), 2.0);
-  for (int row = 0; row < 3; ++row) {
-    double x = r1[row], y = r2[row], z = r3[row];
-    double len = __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(x, x), __dmul_rn(y, y)), __dmul_rn(z, z)));
-    double n = ceil(__ddiv_rn(__ddiv_rn(__dmul_rn(rcut, len), kPiRef), 2.0));
-    if (!(n <= (double)kMaxImage)) {  // also catches NaN
-      atomicOr(flags, kFlagImageLimit);
-      n = (n > 0) ? (double)kMaxImage : 0.0;
-    }
-    si.nabc[row] = (int)n;
+  const double c[3][3] = {{L[0], L[3], L[6]}, {L[1], L[4], L[7]}, {L[2], L[5], L[8]}};
+  double r1[3];
+  crossp_rn(c[1], c[2], r1);
+  const double vol = fabs(__dadd_rn(__dadd_rn(__dmul_rn(c[0][0], r1[0]), __dmul_rn(c[0][1], r1[1])),
+                                    __dmul_rn(c[0][2], r1[2])));
+  // lane 3 a + b: component b of reciprocal vector a
+  double rec = 0.0;
+  {
+    double r2[3], r3[3];
+    crossp_rn(c[2], c[0], r2);
+    crossp_rn(c[0], c[1], r3);
+    const double all[9] = {r1[0], r1[1], r1[2], r2[0], r2[1], r2[2], r3[0], r3[1], r3[2]};
+    double v = all[0];
+#pragma unroll
+    for (int t = 1; t < 9; ++t) v = q == t ? all[t] : v;
+    rec = __dmul_rn(__dmul_rn(__ddiv_rn(v, vol), kPiRef), 2.0);
   }
+  // lane a: |row a| of the three vectors and the image count
+  const int row = q < 3 ? q : 0;
+  const double x = __shfl_sync(0xffffffffu, rec, base + row),
+               y = __shfl_sync(0xffffffffu, rec, base + 3 + row),
+               z = __shfl_sync(0xffffffffu, rec, base + 6 + row);
+  const double len =
+      __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(x, x), __dmul_rn(y, y)), __dmul_rn(z, z)));
+  double n = ceil(__ddiv_rn(__ddiv_rn(__dmul_rn(rcut, len), kPiRef), 2.0));
+  if (!(n <= (double)kMaxImage)) {  // also catches NaN
+    if (live && q < 3) atomicOr(flags, kFlagImageLimit);
+    n = (n > 0) ? (double)kMaxImage : 0.0;
+  }
+  StructInfo &o = out[s];
   // det(lat) as gap_calc.f90:295-297
-  double det = __dadd_rn(
+  const double det = __dadd_rn(
       __dsub_rn(__dmul_rn(L[0], __dsub_rn(__dmul_rn(L[4], L[8]), __dmul_rn(L[5], L[7]))),
                 __dmul_rn(L[1], __dsub_rn(__dmul_rn(L[3], L[8]), __dmul_rn(L[5], L[6])))),
       __dmul_rn(L[2], __dsub_rn(__dmul_rn(L[3], L[7]), __dmul_rn(L[6], L[4]))));
-  si.volume = fabs(det);
-  // inverse of L (rows = lattice vectors): adjugate / det
-  double inv[9];
-  inv[0] = (L[4] * L[8] - L[5] * L[7]) / det;
-  inv[1] = (L[2] * L[7] - L[1] * L[8]) / det;
-  inv[2] = (L[1] * L[5] - L[2] * L[4]) / det;
-  inv[3] = (L[5] * L[6] - L[3] * L[8]) / det;
-  inv[4] = (L[0] * L[8] - L[2] * L[6]) / det;
-  inv[5] = (L[2] * L[3] - L[0] * L[5]) / det;
-  inv[6] = (L[3] * L[7] - L[4] * L[6]) / det;
-  inv[7] = (L[1] * L[6] - L[0] * L[7]) / det;
-  inv[8] = (L[0] * L[4] - L[1] * L[3]) / det;
-  for (int q = 0; q < 9; ++q) si.linv[q] = inv[q];
-  for (int a = 0; a < 3; ++a) {
-    double cl = sqrt(inv[a] * inv[a] + inv[3 + a] * inv[3 + a] + inv[6 + a] * inv[6 + a]);
-    // FP32 fractional coordinates are compared against this bound: margin
-    // for their rounding (|f| < 1e3 keeps the error below 1e-4)
-    si.ext[a] = rcut * cl * (1.0 + 1e-9) + 2e-4;
+  // inverse of L (rows = lattice vectors): adjugate / det, entry q
+  const double adj[9] = {L[4] * L[8] - L[5] * L[7], L[2] * L[7] - L[1] * L[8],
+                         L[1] * L[5] - L[2] * L[4], L[5] * L[6] - L[3] * L[8],
+                         L[0] * L[8] - L[2] * L[6], L[2] * L[3] - L[0] * L[5],
+                         L[3] * L[7] - L[4] * L[6], L[1] * L[6] - L[0] * L[7],
+                         L[0] * L[4] - L[1] * L[3]};
+  double num = adj[0], lq = L[0];
+#pragma unroll
+  for (int t = 1; t < 9; ++t) {
+    num = q == t ? adj[t] : num;
+    lq = q == t ? L[t] : lq;
   }
-  {
-    float lsum = 0.f;
-    for (int q = 0; q < 9; ++q) {
-      si.lat32[q] = (float)si.lat[q];
-      si.latl32[q] = (float)(si.lat[q] - (double)si.lat32[q]);
-      lsum += fabsf(si.lat32[q]);
-    }
-    const float rs = (float)rcut + 2.5e-4f * lsum + 1e-3f;
-    si.r2max32 = rs * rs;
-    si.rc2_32 = (float)(rcut * rcut);
-    for (int a = 0; a < 3; ++a) si.ext32[a] = (float)si.ext[a];
-    si.single = (2.f * si.ext32[0] < 1.f) & (2.f * si.ext32[1] < 1.f) & (2.f * si.ext32[2] < 1.f);
-  }
-  si.a0 = atom_off[s];
-  si.na = atom_off[s + 1] - atom_off[s];
+  const double inv = num / det;
+  // lane a: extent of axis a.  FP32 fractional coordinates are compared
+  // against this bound: margin for their rounding (|f| < 1e3 keeps the error
+  // below 1e-4)
+  const double i0 = __shfl_sync(0xffffffffu, inv, base + row),
+               i1 = __shfl_sync(0xffffffffu, inv, base + 3 + row),
+               i2 = __shfl_sync(0xffffffffu, inv, base + 6 + row);
+  const double ext = rcut * sqrt(i0 * i0 + i1 * i1 + i2 * i2) * (1.0 + 1e-9) + 2e-4;
+  const float ext32 = (float)ext;
+  const float e0 = __shfl_sync(0xffffffffu, ext32, base),
+              e1 = __shfl_sync(0xffffffffu, ext32, base + 1),
+              e2 = __shfl_sync(0xffffffffu, ext32, base + 2);
+  const int single = (2.f * e0 < 1.f) & (2.f * e1 < 1.f) & (2.f * e2 < 1.f);
   // bins of fractional width >= ext (+ 1e-3 for the FP32 coordinates of the
   // binning) when the cell is at least 3 bins wide on every axis
-  si.nb[0] = si.nb[1] = si.nb[2] = 0;
-  si.bin0 = 0;
-  if (allow_bins && si.na >= kBinMinAtoms) {
-    int nb[3];
-    bool ok = true;
-    long prod = 1;
-    for (int a = 0; a < 3; ++a) {
-      nb[a] = (int)floor(1.0 / (si.ext[a] + 1e-3));
-      if (nb[a] > 64) nb[a] = 64;
-      if (nb[a] < 3) ok = false;
-      prod *= nb[a];
-    }
-    if (ok && prod <= si.na)
-      for (int a = 0; a < 3; ++a) si.nb[a] = nb[a];
+  const int a0 = atom_off[s], na = atom_off[s + 1] - a0;
+  int nb = 0;
+  if (allow_bins && na >= kBinMinAtoms) {
+    nb = (int)floor(1.0 / (ext + 1e-3));
+    if (nb > 64) nb = 64;
   }
-  // which of the two neighbour kernels has work (the other returns at once)
-  if (si.nb[0] == 0) atomicOr(flags + (si.single ? 4 : 3), 1);
-  out[s] = si;
+  const int b0 = __shfl_sync(0xffffffffu, nb, base), b1 = __shfl_sync(0xffffffffu, nb, base + 1),
+            b2 = __shfl_sync(0xffffffffu, nb, base + 2);
+  const bool binned = b0 >= 3 && b1 >= 3 && b2 >= 3 && (long)b0 * b1 * b2 <= na;
+  if (!live) return;
+  if (q < 9) {
+    const float hi = (float)lq;
+    o.lat[q] = lq;
+    o.linv[q] = inv;
+    o.lat32[q] = hi;
+    o.latl32[q] = (float)(lq - (double)hi);
+  }
+  if (q < 3) {
+    o.nabc[q] = (int)n;
+    o.ext[q] = ext;
+    o.ext32[q] = ext32;
+    o.nb[q] = binned ? nb : 0;
+  }
+  if (q == 0) {
+    float lsum = 0.f;
+    for (int t = 0; t < 9; ++t) lsum += fabsf((float)L[t]);
+    const float rs = (float)rcut + 2.5e-4f * lsum + 1e-3f;
+    o.r2max32 = rs * rs;
+    o.rc2_32 = (float)(rcut * rcut);
+    o.volume = fabs(det);
+    o.single = single;
+    o.a0 = a0;
+    o.na = na;
+    o.bin0 = 0;
+    // which of the two neighbour kernels has work (the other returns at once)
+    if (!binned) atomicOr(flags + (single ? 4 : 3), 1);
+  }
 }
 
 // ---- spatial bins of large cells -------------------------------------------
@@ -864,9 +890,11 @@ int grid_for_warps(int nwarps_needed) {
 
 void launch_prep(const gapgb_model *m, Workspace &ws, int S, int N, const int *d_atom_off,
                  const int *d_species, const double *d_lat, const double *d_pos, double rcut,
-                 cudaStream_t st, bool allow_bins) {
-  k_prep_struct<<<(S + 127) / 128, 128, 0, st>>>(S, d_atom_off, d_lat, rcut, allow_bins ? 1 : 0,
-                                                 ws.sinfo, ws.d_flags);
+                 cudaStream_t st, bool allow_bins, bool lattice) {
+  constexpr int per = 128 / kPrepLanes;
+  if (lattice)
+    k_prep_struct<<<(S + per - 1) / per, 128, 0, st>>>(S, d_atom_off, d_lat, rcut,
+                                                       allow_bins ? 1 : 0, ws.sinfo, ws.d_flags);
   k_prep_atoms<<<(N + 255) / 256, 256, 0, st>>>(N, S, d_atom_off, d_species, d_pos, m->d_sf,
                                                  ws.sinfo, ws.atom_struct, ws.apos, ws.frac32,
                                                  ws.pos2f, ws.d_flags);
