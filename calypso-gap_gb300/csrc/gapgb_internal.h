@@ -462,11 +462,16 @@ bool grow_scratch(const gapgb_model *m, void **p, size_t *have, size_t bytes, cu
 gapgb_status g64_prepare(gapgb_model *m, bool refresh = false);
 template <typename TG>
 bool launch_gpr64(const gapgb_model *m, Workspace &ws, int N, cudaStream_t st);
+bool launch_phi64(const gapgb_model *m, Workspace &ws, int N, int S, int Mf, const int *d_off,
+                  const double *G, double *phi, cudaStream_t st);
+bool launch_kmm64(const gapgb_model *m, Workspace &ws, int Mf, double *A, cudaStream_t st);
 // wacsf64.cu: the FP64 descriptor kernels of the usual SF sets
 gapgb_status w64_prepare(gapgb_model *m);
 bool w64_applies(const gapgb_model *m, Workspace &ws, int capS, cudaStream_t st);
 void launch_w64_fwd(const gapgb_model *m, Workspace &ws, int N, int cap, int capS, cudaStream_t st);
 void launch_w64_bwd(const gapgb_model *m, Workspace &ws, int N, int cap, int capS, cudaStream_t st);
+bool launch_w64_jac(const gapgb_model *m, Workspace &ws, int N, int cap, int capS, double *J,
+                    cudaStream_t st);
 // whether the FP32 gradient kernel of this model scatters the forces itself
 // (the reverse slots are then not needed)
 bool bwd_scatters_forces(const gapgb_model *m);

@@ -702,6 +702,43 @@ __global__ void __launch_bounds__(kR)
   dedg[(size_t)i * D + d] = (TG)(re == kRowNaN ? e : -unscale[d] * g);
 }
 
+// phi[s][k] += sum over the structures' atoms within [i0, i1) of K_ik (W: the
+// kernel values of the row tiles from i0 on); the first part of a structure
+// sets.  A warp per (structure, point), lanes over rows: fixed order.
+__global__ void __launch_bounds__(256)
+    k_g64_phi(int i0, int i1, int Mp, int Mf, const int *__restrict__ off,
+              const double *__restrict__ W, double *__restrict__ phi) {
+  const int s = blockIdx.y, lane = threadIdx.x & 31;
+  const int k = blockIdx.x * 8 + (threadIdx.x >> 5);
+  const int a0 = max(off[s], i0), a1 = min(off[s + 1], i1);
+  if (k >= Mf || (a0 >= a1 && off[s] != off[s + 1])) return;
+  double v = 0.0;
+  for (int i = a0 + lane; i < a1; i += 32)
+    v += W[((size_t)((i - i0) / kR) * Mp + k) * kR + (i - i0) % kR];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  if (lane == 0) {
+    double *p = phi + (size_t)s * Mf + k;
+    *p = off[s] >= i0 ? v : *p + v;
+  }
+}
+
+// A[i0 + r][k] = K(m_r, m_k) of one row tile (rows and columns below M; the
+// padded columns zero), transposed through shared memory
+__global__ void __launch_bounds__(256)
+    k_g64_kmm(int M, int i0, int Mp, int Mf, const double *__restrict__ W, double *__restrict__ A) {
+  __shared__ double t[32][33];
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const int r0 = blockIdx.y * 32, k0 = blockIdx.x * 32;  // r0 within the chunk's rows
+  for (int q = ty; q < 32; q += 8)
+    t[q][tx] = W[((size_t)(r0 / kR) * Mp + k0 + q) * kR + r0 % kR + tx];
+  __syncthreads();
+  for (int q = ty; q < 32; q += 8) {
+    const int r = i0 + r0 + q, k = k0 + tx;
+    if (r < M && k < Mf) A[(size_t)r * Mf + k] = k < M ? t[tx][q] : 0.0;
+  }
+}
+
 size_t smem1(int kd) {
   return (size_t)kS1 * slice1(kd) + nbuf1(kd) * tile1(kd) + kExpN * 8 + 4 * kT1 * 16 + 128 + 1024;
 }
@@ -870,6 +907,57 @@ bool launch_gpr64(const gapgb_model *m, Workspace &ws, int N, cudaStream_t st) {
         rowexp, (const int *)(p + g.eD), xh, (const double *)(p + g.unscale), ws.e, (TG *)ws.dedg);
   }
   return true;
+}
+
+// Kernel values without coefficients, for the fit: row tiles in chunks.
+// use(first row, row tiles, W) enqueues what reads them.
+template <typename F>
+static bool g64_kernel_values(const gapgb_model *m, Workspace &ws, int N, const double *X,
+                              cudaStream_t st, F use) {
+  if (!m->d_g64) return false;
+  const int M = m->host.M, D = m->host.D;
+  const G64 g = g64_layout(M, D);
+  const G64Run r = g64_run(g, N, D);
+  if (!grow_scratch(m, &ws.g64_scratch, &ws.g64_bytes, r.bytes, st)) return false;
+  const unsigned char *p = m->d_g64;
+  unsigned char *q = (unsigned char *)ws.g64_scratch;
+  Row *row = (Row *)(q + r.row);
+  k_g64_atoms<double><<<r.tiles * (kR / 8), 128, 0, st>>>(
+      N, D, g.KD, X, (const double *)(p + g.mu), (const double *)(p + g.scale),
+      (double *)(q + r.xh), q + r.img, row, (int *)(q + r.rowexp));
+  auto fw = g.KD == 64 ? k_g64_w<64> : k_g64_w<80>;
+  kernel_smem((const void *)fw, (int)smem1(g.KD), true);
+  for (int c0 = 0; c0 < r.tiles; c0 += r.ct) {
+    const int ct = std::min(r.ct, r.tiles - c0);
+    fw<<<dim3(ct, r.sa), kThreads, smem1(g.KD), st>>>(
+        g.nt1, g.Mp, q + r.img + (size_t)c0 * kS1 * slice1(g.KD), row + (size_t)c0 * kR,
+        p + g.img1, (const Col *)(p + g.col), (const u64 *)(p + g.tab), (double *)(q + r.W),
+        nullptr, ws.d_flags);
+    use(c0 * kR, ct, (const double *)(q + r.W));
+  }
+  return true;
+}
+
+// phi[S][Mf]: sums of the kernel values over each structure's atoms
+bool launch_phi64(const gapgb_model *m, Workspace &ws, int N, int S, int Mf, const int *d_off,
+                  const double *G, double *phi, cudaStream_t st) {
+  const int Mp = g64_layout(m->host.M, m->host.D).Mp;
+  return g64_kernel_values(m, ws, N, G, st, [&](int i0, int ct, const double *W) {
+    k_g64_phi<<<dim3((Mf + 7) / 8, S), 256, 0, st>>>(i0, std::min(N, i0 + ct * kR), Mp, Mf, d_off,
+                                                     W, phi);
+  });
+}
+
+// A[M][Mf] = K_MM
+bool launch_kmm64(const gapgb_model *m, Workspace &ws, int Mf, double *A, cudaStream_t st) {
+  const int M = m->host.M;
+  const G64 g = g64_layout(M, m->host.D);
+  if (!m->d_g64) return false;
+  return g64_kernel_values(m, ws, M, (const double *)(m->d_g64 + g.mm), st,
+                           [&](int i0, int ct, const double *W) {
+                             k_g64_kmm<<<dim3((Mf + 31) / 32, ct * (kR / 32)), 256, 0, st>>>(
+                                 M, i0, g.Mp, Mf, W, A);
+                           });
 }
 
 template bool launch_gpr64<double>(const gapgb_model *, Workspace &, int, cudaStream_t);

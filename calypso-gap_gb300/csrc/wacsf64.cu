@@ -808,11 +808,156 @@ void fc_series(double rc, double *kv, double *c) {
   for (int m = 0; m < kFcN; ++m) c[m] = a[m].h;
 }
 
+// The Jacobian J[i][slot][xyz][d] = dG_id / dp_slot of atoms [0, N): what the
+// gradient contracts with one dE/dG, kept for contractions with many (the
+// force rows of a fit).  One block per atom; a pair's scalars (as in
+// k_w64_bwd, one triple per angular SF of the group) pass through the block's
+// scratch and are gathered by thread = (slot, SF).
+template <int NAL, int DEG>
+__global__ void __launch_bounds__(kBlk)
+    k_w64_jac(int N, int cap, int capS, const int *__restrict__ cnt,
+              const double4 *__restrict__ xyzr, const int *__restrict__ nj,
+              const double4 *__restrict__ apos, const float4 *__restrict__ d32,
+              const W64Tab *__restrict__ tab, const __grid_constant__ W64Fc fc,
+              const double *__restrict__ expt, double *__restrict__ J, double4 *scr, size_t nsc,
+              int namax) {
+  extern __shared__ __align__(32) unsigned char smraw[];
+  const W64Tab &t = *tab;
+  const Lay l = layout(capS, t.nrc, 0);
+  const View s = view(smraw, l);
+  const int tid = threadIdx.x, lane = tid & 31;
+  for (int q = tid; q < kExpN; q += kBlk) reinterpret_cast<double *>(smraw)[q] = expt[q];
+  for (int i = blockIdx.x; i < N; i += gridDim.x) {
+    __syncthreads();
+    const int P = stage<true>(s, t, fc, i, cap, capS, cnt, xyzr, nj, apos, d32, true);
+    double *Ji = J + (size_t)i * capS * 3 * t.D;
+    __syncthreads();
+    for (int e = tid; e < P * 3 * t.D; e += kBlk) Ji[e] = 0.0;
+    __syncthreads();
+    for (int e = tid; e < P * t.nrad; e += kBlk) {
+      const int q = e / t.nrad, a = e - q * t.nrad;
+      const double2 f = s.fc[(size_t)t.rad_rc[a] * capS + q], b = s.B[q];
+      if ((__double2hiint(f.x) | __double2hiint(f.y)) == 0) continue;  // beyond the cutoff
+      const double4 d = s.A[q];
+      const double al = t.rad_alpha[a], u = s.R[q] - t.rad_rs[a];
+      const double v = exp_tab(-al, -al * kPerExp, u * u, s.T) *
+                       fma(-2.0 * al * (u * b.x), f.x, f.y);
+      const double dd[3] = {d.x, d.y, d.z};
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        double *o = Ji + ((size_t)q * 3 + c) * t.D + t.rad_d[a];
+        o[0] = v * dd[c];
+        o[t.nsf] = v * b.y * dd[c];
+      }
+    }
+    for (int g = 0; g < t.ngrp; ++g) {
+      __syncthreads();
+      int n;
+      const int np = build_pairs<true>(s, t, g, P, n);
+      const int rci = t.grp_rc[g], s0 = t.grp_start[g], na = t.grp_start[g + 1] - s0;
+      const double rc2 = t.rc2[rci], kv = t.kv[rci], kd = t.kd[rci];
+      const double2 *f = s.fc + (size_t)rci * capS;
+      double4 *sc = scr + (size_t)blockIdx.x * nsc;
+      for (int p0 = 0; p0 < np; p0 += kUnit) {
+        const int p1 = min(np, p0 + kUnit);
+        __syncthreads();
+        expand(s, n, p0, p1);
+        for (int p = p0 + tid; p - lane < p1; p += kBlk) {
+          if (p >= p1) continue;
+          const unsigned jk = s.list[p - p0];
+          const int j = jk & 0xffff, k = jk >> 16;
+          const double4 aj = s.A[j], ak = s.A[k];
+          const double cx = aj.x - ak.x, cy = aj.y - ak.y, cz = aj.z - ak.z;
+          const double c2 = fma(cx, cx, fma(cy, cy, cz * cz));
+          const double2 bj = s.B[j], bk = s.B[k], fj = f[j], fk = f[k];
+          double fcc, fcd;
+          fc_poly2(fc.c[rci], fma(c2, kv, -1.0), fcc, fcd);
+          const bool in = c2 <= rc2;
+          fcc = in ? fcc : 0.0;
+          fcd = in ? fcd * kd : 0.0;
+          const double iab = bj.x * bk.x, sab = aj.w + ak.w;
+          const double cosv = fma(-0.5, c2, sab) * iab, s3 = fma(2.0, sab, c2);
+          double E[NAL];
+#pragma unroll
+          for (int q = 0; q < NAL; ++q) {
+            const double al = -t.alpha[g][q];
+            E[q] = in ? exp_tab(al, al * kPerExp, s3, s.T) : 0.0;
+          }
+          const double fab = fj.x * fk.x, F = fab * fcc;
+          const double ca = fma(-cosv, bj.x * bj.x, iab), cb = fma(-cosv, bk.x * bk.x, iab);
+          const double ga = fcc * fk.x * fj.y, gb = fcc * fj.x * fk.y, gc = fab * fcd;
+          for (int a = 0; a < na; ++a) {
+            const double *m = t.mono[s0 + a];
+            double pv = m[DEG], pd = 0.0;
+#pragma unroll
+            for (int o = DEG - 1; o >= 0; --o) {
+              pd = fma(pd, cosv, pv);
+              pv = fma(pv, cosv, m[o]);
+            }
+            const int q = t.ang_q[s0 + a];
+            double e = E[0];
+#pragma unroll
+            for (int z = 1; z < NAL; ++z) e = q == z ? E[z] : e;
+            const double SQ = e * pv, SP = e * pd, SU = 2.0 * t.alpha[g][q] * SQ;
+            const double c3 = fma(F, fma(-SP, iab, -SU), SQ * gc);
+            const double c1 = fma(F, fma(SP, ca, -SU), SQ * ga) + c3;
+            const double cc = fma(F, fma(SP, cb, -SU), SQ * gb) + c3;
+            sc[(size_t)p * namax + a] = make_double4(c1, cc, c3, 0.0);
+          }
+        }
+      }
+      __syncthreads();
+      const int W = (n + 31) >> 5;
+      for (int e = tid; e < n * na; e += kBlk) {
+        const int q = e / na, a = e - q * na, wq = q >> 5;
+        const unsigned below = (1u << (q & 31)) - 1u;
+        double x = 0, y = 0, z = 0, o = 0, xw = 0, yw = 0, zw = 0, ow = 0;
+        for (int w = 0; w < W; ++w) {
+          unsigned m = s.mask[q * W + w];
+          int up = s.row[q] + s.pre[q * W + w];
+          while (m) {
+            const int k = 32 * w + __ffs(m) - 1;
+            m &= m - 1;
+            const bool first = k > q;
+            const int pr = first ? up++
+                                 : s.row[k] + s.pre[k * W + wq] + __popc(upper(s, W, k, wq) & below);
+            const double4 v = sc[(size_t)pr * namax + a];
+            const int sk = s.idx[k];
+            const double4 d = s.A[sk];
+            const double wk = s.B[sk].y, c = v.z, own = first ? v.x : v.y;
+            const double cw = c * wk;
+            x = fma(-c, d.x, x), y = fma(-c, d.y, y), z = fma(-c, d.z, z), o += own;
+            xw = fma(-cw, d.x, xw), yw = fma(-cw, d.y, yw), zw = fma(-cw, d.z, zw);
+            ow = fma(own, wk, ow);
+          }
+        }
+        const int sq = s.idx[q], dst = t.ang_d[s0 + a];
+        const double4 d = s.A[sq];
+        const double wq2 = s.B[sq].y;
+        const double v[3] = {fma(o, d.x, x), fma(o, d.y, y), fma(o, d.z, z)};
+        const double vw[3] = {fma(ow, d.x, xw), fma(ow, d.y, yw), fma(ow, d.z, zw)};
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          double *out = Ji + ((size_t)sq * 3 + c) * t.D + dst;
+          out[0] = v[c];
+          out[t.nsf] = wq2 * vw[c];
+        }
+      }
+    }
+  }
+}
+
 // C(n, k) for n <= 4
 double binom(int n, int k) {
   double b = 1.0;
   for (int q = 1; q <= k; ++q) b = b * (n - q + 1) / q;
   return b;
+}
+
+using Jac = decltype(&k_w64_jac<1, 1>);
+template <int NAL>
+Jac pick_jac(int deg) {
+  return deg <= 1 ? k_w64_jac<NAL, 1> : (deg <= 2 ? k_w64_jac<NAL, 2> : k_w64_jac<NAL, 4>);
 }
 
 using Fwd = decltype(&k_w64_fwd<1, 1>);
@@ -1012,6 +1157,25 @@ void launch_w64_bwd(const gapgb_model *m, Workspace &ws, int N, int cap, int cap
                                                 ws.apos, ws.nbr_d32, m->d_w64, m->w64h.fc,
                                                 (double4 *)ws.gslot, ws.wvir, sc, rad, nsc);
   }
+}
+
+// The Jacobians of the batch's atoms into J[N][capS][3][D]; false (nothing
+// launched) when the batch does not take these kernels.
+bool launch_w64_jac(const gapgb_model *m, Workspace &ws, int N, int cap, int capS, double *J,
+                    cudaStream_t st) {
+  if (!w64_applies(m, ws, capS, st)) return false;
+  const W64Tab &t = m->w64h;
+  int na = 1;
+  for (int g = 0; g < t.ngrp; ++g) na = std::max(na, t.grp_start[g + 1] - t.grp_start[g]);
+  const Jac f = t.nal <= 1 ? pick_jac<1>(t.deg) : (t.nal <= 2 ? pick_jac<2>(t.deg) : pick_jac<4>(t.deg));
+  const size_t smem = layout(capS, t.nrc, 0).total, nsc = group_units(capS) * kUnit * na;
+  kernel_smem((const void *)f, (int)smem, true);
+  int gx = std::min(N, device_sms() * kernel_occupancy((const void *)f, kBlk, smem));
+  gx = (int)std::min<size_t>(gx, std::max<size_t>(1, kScratchMax / (nsc * 32)));
+  if (!scratch(m, ws, gx * nsc * 32, st)) return false;
+  f<<<gx, kBlk, smem, st>>>(N, cap, capS, ws.nbr_cnt, ws.nbr_xyz, ws.nbr_j, ws.apos, ws.nbr_d32,
+                            m->d_w64, t.fc, m->d_exp64, J, (double4 *)ws.w64_scratch, nsc, na);
+  return true;
 }
 
 }  // namespace gapgb
