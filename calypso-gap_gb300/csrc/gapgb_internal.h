@@ -219,16 +219,25 @@ inline SFT<T> make_sft(const SFDev &s) {
 // the fc polynomial, radial SFs, and the angular SFs grouped by cutoff, each a
 // combination of moments (bern) and of powers of cos (mono), 2^(1-zeta) included.
 constexpr int kFcN = 12;  // coefficients of the fc polynomial
-struct W64Fc {
-  double c[kMaxRC][kFcN];
+struct W64Cut {
+  unsigned long long c[kFcN];  // fc = sum (-1)^n c_n w^n, units of 2^-61
+  unsigned long long ratio;    // r^2 to w: kv / 2 in units of 2^(-63 - E), rc^2 <= 2^E
+  int top;                     // biased exponent of 2^(E - 1)
 };
+struct W64Fc {
+  W64Cut c[kMaxRC];
+};
+// 2^(j/1024) in units of 2^-63 (gpr64_tc.cu)
+constexpr int kExpN = 1024;
+const unsigned long long *exp2_table();
 struct W64Tab {
   int nsf, D, nrad, nang, nrc, ngrp, nal, deg;  // nal, deg: the kernels' template sizes
   double rc[kMaxRC], rc2[kMaxRC], kv[kMaxRC], kd[kMaxRC];
   int rad_d[kMaxSF], rad_rc[kMaxSF];
-  double rad_alpha[kMaxSF], rad_rs[kMaxSF];
+  // exponents as exp_fix takes them: a = -alpha and 1024 a / ln 2 in two parts
+  double rad_a[kMaxSF], rad_ah[kMaxSF], rad_al[kMaxSF], rad_rs[kMaxSF];
   int grp_rc[kMaxRC], grp_start[kMaxRC + 1];
-  double alpha[kMaxRC][4];
+  double alpha[kMaxRC][4], alpha_h[kMaxRC][4], alpha_l[kMaxRC][4];
   int ang_d[kMaxSF], ang_g[kMaxSF], ang_q[kMaxSF];
   double bern[kMaxSF][5], mono[kMaxSF][5];
   W64Fc fc;  // the cutoffs' polynomials (also passed by value, for the constant bank)
@@ -347,7 +356,7 @@ struct gapgb_model {
   gapgb::SFT<float> sft32h{};          // host copy (kernel selection)
   gapgb::W64Tab w64h{};                // FP64 descriptor kernels' table (wacsf64.cu)
   gapgb::W64Tab *d_w64 = nullptr;
-  double *d_exp64 = nullptr;           // 2^(j/1024)
+  unsigned long long *d_exp64 = nullptr;  // exp2_table
   bool w64_tried = false;              // w64_prepare ran (d_w64 stays null: the set does not qualify)
   double *d_mmt = nullptr;             // M x D, mm / theta (FP64)
   float *d_mmt32 = nullptr;            // M x D, mm / theta (FP32)

@@ -64,7 +64,6 @@ constexpr int kS2 = 8;         // digits of w and m in k_g64_b
 constexpr int kN2 = 64;        // descriptor components per CTA of k_g64_b
 constexpr int kDrain = 4;      // stages between drains of k_g64_b (128 points)
 constexpr int kThreads = 288;  // 8 epilogue / conversion warps and one that issues
-constexpr int kExpN = 1024;
 constexpr int kRowNaN = INT_MAX;
 
 // constants of one sparse point: z's column term in units of 2^-52, the scale
@@ -748,6 +747,24 @@ size_t up256(size_t x) { return (x + 255) / 256 * 256; }
 
 }  // namespace
 
+const u64 *exp2_table() {
+  static const std::vector<u64> T = [] {
+    // 2^(j/1024) in 1.63 fixed point: products of the successive square roots of 2
+    typedef unsigned __int128 u128;
+    std::vector<u64> v(kExpN, (u64)1 << 63);
+    u128 sq = (u128)1 << 127;  // 2 in 2.126
+    for (int b = kExpN / 2; b > 0; b >>= 1) {
+      u64 x = (u64)(std::sqrt((double)(u64)(sq >> 64)) * 4294967296.0);
+      for (int it = 0; it < 3; ++it) x = (u64)(((u128)x + sq / x) >> 1);
+      for (int j = 0; j < kExpN; ++j)
+        if (j & b) v[j] = (u64)(((u128)v[j] * x + ((u128)1 << 62)) >> 63);
+      sq = (u128)x << 63;
+    }
+    return v;
+  }();
+  return T.data();
+}
+
 // device image of a model: layout offsets from m->d_g64
 struct G64 {
   int KD, Mp, nt1, nst, nz;
@@ -797,25 +814,11 @@ gapgb_status g64_prepare(gapgb_model *m, bool refresh) {
       sc[d] = root / h.theta[d];
       sc[up256(8 * (size_t)D) / 8 + d] = 1.0 / (h.theta[d] * root);
     }
-    static const std::vector<u64> T = [] {
-      // 2^(j/1024) in 1.63 fixed point: products of the successive square roots of 2
-      typedef unsigned __int128 u128;
-      std::vector<u64> v(kExpN, (u64)1 << 63);
-      u128 sq = (u128)1 << 127;  // 2 in 2.126
-      for (int b = kExpN / 2; b > 0; b >>= 1) {
-        u64 x = (u64)(std::sqrt((double)(u64)(sq >> 64)) * 4294967296.0);
-        for (int it = 0; it < 3; ++it) x = (u64)(((u128)x + sq / x) >> 1);
-        for (int j = 0; j < kExpN; ++j)
-          if (j & b) v[j] = (u64)(((u128)v[j] * x + ((u128)1 << 62)) >> 63);
-        sq = (u128)x << 63;
-      }
-      return v;
-    }();
     cudaError_t e = cudaMemcpyAsync(p + g.scale, sc.data(), 8 * sc.size(), cudaMemcpyHostToDevice, m->stream);
     if (e == cudaSuccess)
       e = cudaMemcpyAsync(p + g.mm, h.mm.data(), 8 * h.mm.size(), cudaMemcpyHostToDevice, m->stream);
     if (e == cudaSuccess)
-      e = cudaMemcpyAsync(p + g.tab, T.data(), 8 * T.size(), cudaMemcpyHostToDevice, m->stream);
+      e = cudaMemcpyAsync(p + g.tab, exp2_table(), 8 * (size_t)kExpN, cudaMemcpyHostToDevice, m->stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(p + g.emax, 0x80, 16, m->stream);
     const double *mu = (const double *)(p + g.mu), *scale = (const double *)(p + g.scale);
     k_g64_mean<<<D, 256, 0, m->stream>>>(M, D, (const double *)(p + g.mm), (double *)(p + g.mu));

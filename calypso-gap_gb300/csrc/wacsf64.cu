@@ -14,7 +14,10 @@
 //    polynomial of degree 11 in r^2, with fc'(r)/r from its derivative, so neither
 //    the slots nor the pairs take a cosine, and a pair takes no square root
 //    and no division either (every factor is written in r^2 and 1/r_slot);
-//  - exp by a 1024-entry table of 2^(j/1024) and a degree-4 polynomial;
+//  - that polynomial runs in 64-bit fixed point on the integer pipe, and so
+//    does the exponential past its argument reduction (a 1024-entry table of
+//    2^(j/1024) and a degree-4 polynomial): 5 FP64 instructions instead of 10,
+//    and 0 or 1 instead of 12 or 23, with errors below 0.5 and 1 ulp;
 //  - the (1 +- cos)^zeta of a cutoff group are combinations of the products
 //    u^n w^(DEG-n) (u = (1 + cos)/2, w = 1 - u) with non-negative weights: a
 //    pair adds those products, times each alpha's exponential, to moments;
@@ -22,12 +25,14 @@
 //    so a pair needs one Horner pass for value and derivative, and it yields
 //    three scalars (s1 + s3, s2 + s3, s3); a slot's gradient is then
 //    d_q sum(s_own + s3) - sum(s3 d_other), gathered per slot.
-// Per pair of the standard set that is about 80 FP64 instructions for the
-// descriptors and 115 for the gradient, where the generic kernels issue about
+// Per pair of the standard set that is about 60 FP64 instructions for the
+// descriptors and 80 for the gradient, where the generic kernels issue about
 // 520 and 770.  Measured (ncu, both generic kernels -> these, split launches
-// included): 512 alloy atoms (56 slots, 690 pairs each) 520 -> 124 us and
-// 665 -> 191 us; 64 carbon atoms (158 slots, 7 cutoffs) 2380 -> 161 us and
-// 1858 -> 329 us.  The FP64 pipe is 62-70 % busy in the larger launches.
+// included): 512 alloy atoms (56 slots, 690 pairs each) 520 -> 98 us and
+// 665 -> 161 us; 64 carbon atoms (158 slots, 7 cutoffs) 2380 -> 119 us and
+// 1858 -> 277 us; 6.2 k atoms of ragged cells 5444 -> 842 and 10177 -> 1330
+// us, of which the polynomial and the exponential on the integer pipe are the
+// last quarter (1139 and 1691 us with FP64 ones).
 //
 // A block of 4 warps works on one atom.  The pair list of each cutoff group
 // is cut into units of 512 pairs.  Small batches spread an atom's units over
@@ -49,50 +54,75 @@ namespace {
 constexpr int kBlk = 128;        // threads per block (4 warps)
 constexpr int kUnit = 512;       // pairs per unit
 constexpr int kClasses = 8;      // residue classes of units (bounds the split)
-constexpr int kExpN = 1024;      // entries of the 2^(j/1024) table
 
-// fc(r) as a polynomial in v = kv r^2 - 1, -1 <= v <= 1 up to the cutoff
-// (W64Fc::c, formed per cutoff by w64_table), and with its derivative by v.
-// The table is a kernel parameter: its entries are constant-bank operands.
-__device__ __forceinline__ double fc_poly(const double (&c)[kFcN], double v) {
-  double p = c[kFcN - 1];
-#pragma unroll
-  for (int n = kFcN - 2; n >= 0; --n) p = fma(p, v, c[n]);
-  return p;
+typedef unsigned long long u64;
+typedef long long i64;
+
+// x 2^sc as a double, rounded (0 < x < 2^63; otherwise zero)
+__device__ __forceinline__ double fix_double(u64 x, int sc) {
+  const int lz = __clzll((i64)x);
+  const u64 m = x << (lz & 63);
+  const u64 b = ((u64)(uint32_t)(1022 + 63 - lz + sc) << 52) + (m >> 11) + ((m >> 10) & 1);
+  return (i64)x > 0 ? __longlong_as_double((i64)b) : 0.0;
 }
-__device__ __forceinline__ void fc_poly2(const double (&c)[kFcN], double v, double &p, double &d) {
-  p = fma(c[kFcN - 1], v, c[kFcN - 2]);
-  d = c[kFcN - 1];
+
+// w = r^2 / rc^2 (kv r^2 / 2) in units of 2^-64, below one
+__device__ __forceinline__ u64 fc_arg(double r2, const W64Cut &c) {
+  const u64 b = (u64)__double_as_longlong(r2);
+  const int sh = c.top - (int)(b >> 52);
+  const u64 m = ((b & 0xFFFFFFFFFFFFFull) | (1ull << 52)) << 11;
+  const u64 u = sh >= 64 ? 0 : (sh <= 0 ? m : m >> sh);
+  const u64 w = __umul64hi(u, c.ratio);
+  return (w >> 63) || sh < 0 ? ~0ull : w << 1;
+}
+// fc = sum (-1)^n c_n w^n in integer arithmetic (units of 2^-61), and -d fc / dw
+__device__ __forceinline__ double fc_fix(const W64Cut &c, double r2) {
+  const u64 w = fc_arg(r2, c);
+  u64 p = c.c[kFcN - 1];
 #pragma unroll
-  for (int n = kFcN - 3; n >= 0; --n) {
-    d = fma(d, v, p);
-    p = fma(p, v, c[n]);
+  for (int n = kFcN - 2; n >= 0; --n) p = c.c[n] - __umul64hi(w, p);
+  return fix_double(p, -61);
+}
+__device__ __forceinline__ void fc_fix2(const W64Cut &c, double r2, double &f, double &d) {
+  const u64 w = fc_arg(r2, c);
+  u64 p = c.c[kFcN - 1], e = 0;
+#pragma unroll
+  for (int n = kFcN - 2; n >= 0; --n) {
+    e = p - __umul64hi(w, e);
+    p = c.c[n] - __umul64hi(w, p);
   }
+  f = fix_double(p, -61);
+  // past pi (the format's pi is 4e-10 above it) the derivative changes sign
+  d = (i64)e < 0 ? -fix_double(0ull - e, -61) : fix_double(e, -61);
 }
 
-// exp(a b) by table lookup (P. T. P. Tang, "Table-driven implementation of the
-// exponential function in IEEE floating-point arithmetic", ACM TOMS 15, 1989):
-// a b = (1024 n + j) ln2/1024 + r, |r| <= ln2/2048, and e^r - 1 to degree 4
-// (the r^5 term is below 4e-20).  The high part of ln2/1024 has 32 bits, so
-// its multiples are exact and r carries the unrounded product a b.  a1 is
-// a 1024/ln 2.  Outside the normal range, and for NaN, the library's exp.
-constexpr double kPerExp = 1477.3197218702985;  // 1024 / ln 2
-__device__ __forceinline__ double exp_tab(double a, double a1, double b,
-                                          const double *__restrict__ T) {
+// exp(a b), the product unrounded: 1024 a b / ln 2 = k + r with ah + al =
+// 1024 a / ln 2, then 2^(k/1024) from a table (P. T. P. Tang, "Table-driven
+// implementation of the exponential function in IEEE floating-point
+// arithmetic", ACM TOMS 15, 1989) and 2^(r/1024) by a degree-4 polynomial, in
+// integer arithmetic (exp2_fix of gpr64_tc.cu).  Outside the normal range, and
+// for NaN, the library's exp.
+__device__ __forceinline__ double exp_fix(double a, double ah, double al, double b,
+                                          const u64 *__restrict__ T) {
   const double kShift = 6755399441055744.0;  // 1.5 2^52: rounds to an integer in the low word
-  const double kf = fma(a1, b, kShift);
-  const int k = __double2loint(kf);
+  const double kf = fma(ah, b, kShift);
   const double kd = kf - kShift;
   if ((__double2hiint(kd) & 0x7fffffff) >= 0x412feb6c) return exp(a * b);  // |a b| >= 708
-  double r = fma(a, b, -(kd * 0x1.62e42fee00000p-11));
-  r = fma(kd, -0x1.a39ef35793c76p-43, r);
-  const double t = T[k & (kExpN - 1)];
-  const double r2 = r * r;
-  double p = fma(r, 1.0 / 24.0, 1.0 / 6.0);
-  p = fma(p, r, 0.5);
-  p = fma(p, r2, r);
-  const double y = fma(t, p, t);
-  return __hiloint2double(__double2hiint(y) + ((k >> 10) << 20), __double2loint(y));
+  const double r = fma(al, b, fma(ah, b, -kd));  // within one of zero
+  const u64 f = (u64)__double_as_longlong(r + 6.0) & 0xFFFFFFFFFFFFFull;  // (r + 2) 2^50
+  const int k = __double2loint(kf) - 2 + (int)(f >> 50);
+  const u64 t = T[k & (kExpN - 1)];
+  // y = the fraction of 1/1024 times ln 2, in units of 2^-74
+  const u64 y = __umul64hi((f & ((1ull << 50) - 1)) << 14, 0xB17217F7D1CF79ACull);
+  const u64 y2 = __umul64hi(y, y);                         // 2^-84
+  const uint32_t yh = (uint32_t)(y >> 32);                 // 2^-42
+  const uint32_t y3 = __umulhi((uint32_t)(y2 >> 32), yh);  // 2^-62
+  const uint32_t y4 = __umulhi(y3, yh);                    // 2^-72
+  const u64 p = y + (y2 >> 11) +
+                ((u64)(__umulhi(y3, 0x2AAAAAABu) + (__umulhi(y4, 0x0AAAAAABu) >> 10)) << 12);
+  const u64 m = t + (__umul64hi(t, p) >> 10);
+  return __longlong_as_double(
+      (i64)(((u64)(uint32_t)((k >> 10) + 1022) << 52) + ((m + 1024) >> 11)));
 }
 
 // sums v[0..N) over the warp's lanes by halving exchanges: at each step a
@@ -155,7 +185,7 @@ __host__ __device__ inline Lay layout(int capS, int nrc, size_t rest) {
 }
 
 struct View {
-  const double *T;
+  const u64 *T;
   double4 *A;
   double2 *B, *fc;
   double *R;
@@ -167,7 +197,7 @@ struct View {
 };
 __device__ __forceinline__ View view(unsigned char *sm, const Lay &l) {
   View v;
-  v.T = reinterpret_cast<const double *>(sm);
+  v.T = reinterpret_cast<const u64 *>(sm);
   v.A = reinterpret_cast<double4 *>(sm + l.A);
   v.B = reinterpret_cast<double2 *>(sm + l.B);
   v.fc = reinterpret_cast<double2 *>(sm + l.fc);
@@ -202,12 +232,11 @@ __device__ __forceinline__ int stage(const View &s, const W64Tab &t, const W64Fc
     for (int c = 0; c < t.nrc; ++c) {
       double f = 0.0, d = 0.0;
       if (r <= t.rc[c]) {
-        const double v = fma(r * r, t.kv[c], -1.0);
         if (GRAD) {
-          fc_poly2(fc.c[c], v, f, d);
+          fc_fix2(fc.c[c], r * r, f, d);
           d *= t.kd[c];
         } else {
-          f = fc_poly(fc.c[c], v);
+          f = fc_fix(fc.c[c], r * r);
         }
       }
       s.fc[(size_t)c * capS + q] = make_double2(f, d);
@@ -318,7 +347,7 @@ __global__ void __launch_bounds__(kBlk, NAL * (DEG + 1) <= 10 ? 5 : 3)
               const double4 *__restrict__ xyzr, const int *__restrict__ nj,
               const double4 *__restrict__ apos, const float4 *__restrict__ d32,
               const W64Tab *__restrict__ tab, const __grid_constant__ W64Fc fc,
-              const double *__restrict__ expt,
+              const u64 *__restrict__ expt,
               double *__restrict__ G, double *__restrict__ part, int split) {
   constexpr int NB = DEG + 1, NM = 2 * NAL * NB;
   extern __shared__ __align__(32) unsigned char smraw[];
@@ -329,7 +358,7 @@ __global__ void __launch_bounds__(kBlk, NAL * (DEG + 1) <= 10 ? 5 : 3)
   double *S = wpart + 4 * NM;                                      // [group][class][NM]
   double *rp = S + (size_t)t.ngrp * kClasses * NM;                 // [2][kBlk]
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  for (int q = tid; q < kExpN; q += kBlk) reinterpret_cast<double *>(smraw)[q] = expt[q];
+  for (int q = tid; q < kExpN; q += kBlk) reinterpret_cast<u64 *>(smraw)[q] = expt[q];
   const int y = blockIdx.y;
   for (int i = blockIdx.x; i < N; i += gridDim.x) {
     __syncthreads();
@@ -343,11 +372,11 @@ __global__ void __launch_bounds__(kBlk, NAL * (DEG + 1) <= 10 ? 5 : 3)
       const int ng = kBlk / t.nrad, sr = tid % t.nrad, gr = tid / t.nrad;
       double acc = 0.0, accw = 0.0;
       if (gr < ng) {
-        const double al = t.rad_alpha[sr], rs = t.rad_rs[sr];
+        const double al = t.rad_a[sr], ah = t.rad_ah[sr], alo = t.rad_al[sr], rs = t.rad_rs[sr];
         const double2 *f = s.fc + (size_t)t.rad_rc[sr] * capS;
         for (int q = gr; q < P; q += ng) {
           const double fq = f[q].x, u = s.R[q] - rs;
-          const double e = exp_tab(-al, -al * kPerExp, u * u, s.T);
+          const double e = exp_fix(al, ah, alo, u * u, s.T);
           const double v = __double2hiint(fq) != 0 ? e * fq : 0.0;  // beyond the cutoff: zero
           acc += v;
           accw = fma(v, s.B[q].y, accw);
@@ -372,13 +401,14 @@ __global__ void __launch_bounds__(kBlk, NAL * (DEG + 1) <= 10 ? 5 : 3)
       int n;
       const int np = build_pairs<false>(s, t, g, P, n);
       const int rci = t.grp_rc[g];
-      const double rc2 = t.rc2[rci], kv = t.kv[rci];
+      const i64 rc2 = __double_as_longlong(t.rc2[rci]);
       const double2 *f = s.fc + (size_t)rci * capS;
-      double al[NAL], al1[NAL];
+      double al[NAL], ah[NAL], alo[NAL];
 #pragma unroll
       for (int q = 0; q < NAL; ++q) {
-        al[q] = -t.alpha[g][q];
-        al1[q] = al[q] * kPerExp;
+        al[q] = t.alpha[g][q];
+        ah[q] = t.alpha_h[g][q];
+        alo[q] = t.alpha_l[g][q];
       }
       const int nu = (np + kUnit - 1) / kUnit;
       for (int u = 0; u < nu; ++u) {
@@ -397,8 +427,8 @@ __global__ void __launch_bounds__(kBlk, NAL * (DEG + 1) <= 10 ? 5 : 3)
           const double cx = aj.x - ak.x, cy = aj.y - ak.y, cz = aj.z - ak.z;
           const double c2 = fma(cx, cx, fma(cy, cy, cz * cz));
           const double2 bj = s.B[j], bk = s.B[k];
-          double fcc = fc_poly(fc.c[rci], fma(c2, kv, -1.0));
-          const bool in = live && c2 <= rc2;  // else exactly zero
+          double fcc = fc_fix(fc.c[rci], c2);
+          const bool in = live && __double_as_longlong(c2) <= rc2;  // else exactly zero
           fcc = in ? fcc : 0.0;
           // costheta = (rij^2 + rik^2 - rjk^2) / (2 rij rik) (wacsf.f90:271-273)
           const double sab = aj.w + ak.w;
@@ -425,7 +455,7 @@ __global__ void __launch_bounds__(kBlk, NAL * (DEG + 1) <= 10 ? 5 : 3)
           }
 #pragma unroll
           for (int q = 0; q < NAL; ++q) {
-            const double ef = in ? exp_tab(al[q], al1[q], s3, s.T) * F : 0.0;
+            const double ef = in ? exp_fix(al[q], ah[q], alo[q], s3, s.T) * F : 0.0;
             const double efw = ef * wjk;
 #pragma unroll
             for (int n = 0; n < NB; ++n) {
@@ -591,7 +621,7 @@ __global__ void __launch_bounds__(kBlk, 4)
               const double4 *__restrict__ xyzr, const int *__restrict__ nj,
               const double4 *__restrict__ apos, const float4 *__restrict__ d32,
               const W64Tab *__restrict__ tab, const __grid_constant__ W64Fc fc,
-              const double *__restrict__ expt, const double *__restrict__ dedg,
+              const u64 *__restrict__ expt, const double *__restrict__ dedg,
               double4 *__restrict__ gslot, double *__restrict__ wvir, double4 *scr,
               double *__restrict__ rad, size_t nsc, int split) {
   constexpr int NB = DEG + 1;
@@ -604,7 +634,7 @@ __global__ void __launch_bounds__(kBlk, 4)
   double *sU = dg + t.D;                                                  // [2][NAL][NB]
   double *vir = sU + 2 * NAL * NB;                                        // [4][9]
   const int tid = threadIdx.x, lane = tid & 31;
-  for (int q = tid; q < kExpN; q += kBlk) reinterpret_cast<double *>(smraw)[q] = expt[q];
+  for (int q = tid; q < kExpN; q += kBlk) reinterpret_cast<u64 *>(smraw)[q] = expt[q];
   const int y = blockIdx.y;
   for (int i = blockIdx.x; i < N; i += gridDim.x) {
     __syncthreads();
@@ -621,15 +651,15 @@ __global__ void __launch_bounds__(kBlk, 4)
         for (int a = 0; a < t.nrad; ++a) {
           const double2 f = s.fc[(size_t)t.rad_rc[a] * capS + q];
           if ((__double2hiint(f.x) | __double2hiint(f.y)) == 0) continue;  // beyond the cutoff
-          const double al = t.rad_alpha[a], rs = t.rad_rs[a];
+          const double al = t.rad_a[a], rs = t.rad_rs[a];
           double u2 = r2, ur = 1.0;
           if (rs != 0.0) {  // uniform over the block
             const double u = r - rs;
             u2 = u * u;
             ur = u * b.x;
           }
-          const double e = exp_tab(-al, -al * kPerExp, u2, s.T);
-          const double g = fma(-2.0 * al * ur, f.x, f.y);
+          const double e = exp_fix(al, t.rad_ah[a], t.rad_al[a], u2, s.T);
+          const double g = fma(2.0 * al * ur, f.x, f.y);
           sum = fma(fma(dg[t.rad_d[a] + t.nsf], b.y, dg[t.rad_d[a]]) * e, g, sum);
         }
         if (split > 1) rad[(size_t)i * capS + q] = sum;
@@ -641,7 +671,8 @@ __global__ void __launch_bounds__(kBlk, 4)
       int n;
       const int np = build_pairs<true>(s, t, g, P, n);
       const int rci = t.grp_rc[g];
-      const double rc2 = t.rc2[rci], kv = t.kv[rci], kd = t.kd[rci];
+      const double kd = t.kd[rci];
+      const i64 rc2 = __double_as_longlong(t.rc2[rci]);
       const double2 *f = s.fc + (size_t)rci * capS;
       // dE/dG contracted onto polynomials in cos: cell (weighting, alpha, power)
       for (int c = tid; c < 2 * NAL * NB; c += kBlk) {
@@ -651,11 +682,12 @@ __global__ void __launch_bounds__(kBlk, 4)
           if (t.ang_q[a] == q) v = fma(t.mono[a][m], dg[t.ang_d[a] + (h ? t.nsf : 0)], v);
         sU[c] = v;
       }
-      double al[NAL], al1[NAL];
+      double al[NAL], ah[NAL], alo[NAL];
 #pragma unroll
       for (int q = 0; q < NAL; ++q) {
-        al[q] = -t.alpha[g][q];
-        al1[q] = al[q] * kPerExp;
+        al[q] = t.alpha[g][q];
+        ah[q] = t.alpha_h[g][q];
+        alo[q] = t.alpha_l[g][q];
       }
       __syncthreads();
       double4 *sc = split > 1 ? scr + (size_t)i * nsc + (size_t)u0 * kUnit
@@ -675,9 +707,9 @@ __global__ void __launch_bounds__(kBlk, 4)
           const double c2 = fma(cx, cx, fma(cy, cy, cz * cz));
           const double2 bj = s.B[j], bk = s.B[k], fj = f[j], fk = f[k];
           double fcc, fcd;
-          fc_poly2(fc.c[rci], fma(c2, kv, -1.0), fcc, fcd);
+          fc_fix2(fc.c[rci], c2, fcc, fcd);
           fcd *= kd;
-          const bool in = live && c2 <= rc2;
+          const bool in = live && __double_as_longlong(c2) <= rc2;
           fcc = in ? fcc : 0.0;
           fcd = in ? fcd : 0.0;
           const double iab = bj.x * bk.x;
@@ -688,7 +720,7 @@ __global__ void __launch_bounds__(kBlk, 4)
           double SP = 0.0, SQ = 0.0, SU = 0.0;
 #pragma unroll
           for (int q = 0; q < NAL; ++q) {
-            const double e = in ? exp_tab(al[q], al1[q], s3, s.T) : 0.0;
+            const double e = in ? exp_fix(al[q], ah[q], alo[q], s3, s.T) : 0.0;
             const double *U0 = sU + q * NB, *U1 = sU + (NAL + q) * NB;
             double pv = fma(wjk, U1[DEG], U0[DEG]), pd = 0.0;
 #pragma unroll
@@ -776,15 +808,18 @@ DD dd_div(DD a, double b) {
   return dd_sum(q, r / b);
 }
 
-// fc(r) = (cos(k r) + 1) / 2, k = pi / rc, in powers of v = kv r^2 - 1, with
-// kv = 2 / rc^2 cut to 24 bits (so that kv itself brings no error, and v stays
-// within 1 + 2^-23): the power series of cos(sqrt(t)), t = w (1 + v) with
-// w = k^2 / kv, expanded in v to degree 18 and economised to degree 11 by
-// Chebyshev polynomials.  Coefficients rounded once; the result is within
-// 2e-17 of fc, and its derivative within 5e-17.
-void fc_series(double rc, double *kv, double *c) {
+// fc(r) = (cos(k r) + 1) / 2, k = pi / rc, in powers of w = kv r^2 / 2, with
+// kv = 2 / rc^2 cut down to 24 bits (so that kv itself brings no error, and w
+// stays at most 1): the power series of cos(sqrt(t)), t = (2 k^2 / kv) w,
+// in powers of v = 2 w - 1 to degree 18, economised to degree 11 by Chebyshev
+// polynomials (largest error 2e-17, the derivative's 5e-17), then in powers of
+// w, whose signs alternate.  Coefficients in units of 2^-61.
+void fc_series(double rc, double *kv, W64Cut *cut) {
   const double k = kPiRef / rc;
-  *kv = (double)(float)(2.0 / (rc * rc));
+  const double k2 = 2.0 / (rc * rc);
+  float kf = (float)k2;
+  if ((double)kf > k2) kf = std::nextafter(kf, 0.f);
+  *kv = (double)kf;
   constexpr int kDeg = 18, kTerms = 28;
   const DD w = dd_div(dd_mul({k, 0.0}, {k, 0.0}), *kv);
   DD a[kDeg + 1] = {};
@@ -805,7 +840,22 @@ void fc_series(double rc, double *kv, double *c) {
     const DD q = dd_div(a[n], -T[n][n]);
     for (int m = 0; m < n; ++m) a[m] = dd_add(a[m], dd_mul(q, {T[n][m], 0.0}));
   }
-  for (int m = 0; m < kFcN; ++m) c[m] = a[m].h;
+  // v = 2 w - 1: coefficient of w^m is sum_n a_n C(n, m) 2^m (-1)^(n - m)
+  double bin[kFcN][kFcN] = {};
+  for (int n = 0; n < kFcN; ++n)
+    for (int m = 0; m <= n; ++m) bin[n][m] = m == 0 || m == n ? 1.0 : bin[n - 1][m - 1] + bin[n - 1][m];
+  for (int m = 0; m < kFcN; ++m) {
+    DD c = {0.0, 0.0};
+    for (int n = m; n < kFcN; ++n)
+      c = dd_add(c, dd_mul(a[n], {std::ldexp(bin[n][m], m) * ((n & 1) ? -1.0 : 1.0), 0.0}));
+    // times (-1)^(n - m) (-1)^m = (-1)^n: the alternating form's coefficient
+    cut->c[m] = (unsigned long long)((__int128)std::ldexp(c.h, 61) + (__int128)std::llround(std::ldexp(c.l, 61)));
+  }
+  // 2^(E - 1) < rc^2 <= 2^E; kv / 2 in units of 2^(-63 - E)
+  int E;
+  if (std::frexp(2.0 / *kv, &E) == 0.5) --E;  // rc^2 a power of two
+  cut->top = E - 1 + 1023;
+  cut->ratio = (unsigned long long)std::ldexp(*kv * 0.5, E + 63);
 }
 
 // The Jacobian J[i][slot][xyz][d] = dG_id / dp_slot of atoms [0, N): what the
@@ -819,14 +869,14 @@ __global__ void __launch_bounds__(kBlk)
               const double4 *__restrict__ xyzr, const int *__restrict__ nj,
               const double4 *__restrict__ apos, const float4 *__restrict__ d32,
               const W64Tab *__restrict__ tab, const __grid_constant__ W64Fc fc,
-              const double *__restrict__ expt, double *__restrict__ J, double4 *scr, size_t nsc,
+              const u64 *__restrict__ expt, double *__restrict__ J, double4 *scr, size_t nsc,
               int namax) {
   extern __shared__ __align__(32) unsigned char smraw[];
   const W64Tab &t = *tab;
   const Lay l = layout(capS, t.nrc, 0);
   const View s = view(smraw, l);
   const int tid = threadIdx.x, lane = tid & 31;
-  for (int q = tid; q < kExpN; q += kBlk) reinterpret_cast<double *>(smraw)[q] = expt[q];
+  for (int q = tid; q < kExpN; q += kBlk) reinterpret_cast<u64 *>(smraw)[q] = expt[q];
   for (int i = blockIdx.x; i < N; i += gridDim.x) {
     __syncthreads();
     const int P = stage<true>(s, t, fc, i, cap, capS, cnt, xyzr, nj, apos, d32, true);
@@ -839,9 +889,9 @@ __global__ void __launch_bounds__(kBlk)
       const double2 f = s.fc[(size_t)t.rad_rc[a] * capS + q], b = s.B[q];
       if ((__double2hiint(f.x) | __double2hiint(f.y)) == 0) continue;  // beyond the cutoff
       const double4 d = s.A[q];
-      const double al = t.rad_alpha[a], u = s.R[q] - t.rad_rs[a];
-      const double v = exp_tab(-al, -al * kPerExp, u * u, s.T) *
-                       fma(-2.0 * al * (u * b.x), f.x, f.y);
+      const double al = t.rad_a[a], u = s.R[q] - t.rad_rs[a];
+      const double v = exp_fix(al, t.rad_ah[a], t.rad_al[a], u * u, s.T) *
+                       fma(2.0 * al * (u * b.x), f.x, f.y);
       const double dd[3] = {d.x, d.y, d.z};
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
@@ -855,7 +905,8 @@ __global__ void __launch_bounds__(kBlk)
       int n;
       const int np = build_pairs<true>(s, t, g, P, n);
       const int rci = t.grp_rc[g], s0 = t.grp_start[g], na = t.grp_start[g + 1] - s0;
-      const double rc2 = t.rc2[rci], kv = t.kv[rci], kd = t.kd[rci];
+      const double kd = t.kd[rci];
+      const i64 rc2 = __double_as_longlong(t.rc2[rci]);
       const double2 *f = s.fc + (size_t)rci * capS;
       double4 *sc = scr + (size_t)blockIdx.x * nsc;
       for (int p0 = 0; p0 < np; p0 += kUnit) {
@@ -871,18 +922,16 @@ __global__ void __launch_bounds__(kBlk)
           const double c2 = fma(cx, cx, fma(cy, cy, cz * cz));
           const double2 bj = s.B[j], bk = s.B[k], fj = f[j], fk = f[k];
           double fcc, fcd;
-          fc_poly2(fc.c[rci], fma(c2, kv, -1.0), fcc, fcd);
-          const bool in = c2 <= rc2;
+          fc_fix2(fc.c[rci], c2, fcc, fcd);
+          const bool in = __double_as_longlong(c2) <= rc2;
           fcc = in ? fcc : 0.0;
           fcd = in ? fcd * kd : 0.0;
           const double iab = bj.x * bk.x, sab = aj.w + ak.w;
           const double cosv = fma(-0.5, c2, sab) * iab, s3 = fma(2.0, sab, c2);
           double E[NAL];
 #pragma unroll
-          for (int q = 0; q < NAL; ++q) {
-            const double al = -t.alpha[g][q];
-            E[q] = in ? exp_tab(al, al * kPerExp, s3, s.T) : 0.0;
-          }
+          for (int q = 0; q < NAL; ++q)
+            E[q] = in ? exp_fix(t.alpha[g][q], t.alpha_h[g][q], t.alpha_l[g][q], s3, s.T) : 0.0;
           const double fab = fj.x * fk.x, F = fab * fcc;
           const double ca = fma(-cosv, bj.x * bj.x, iab), cb = fma(-cosv, bk.x * bk.x, iab);
           const double ga = fcc * fk.x * fj.y, gb = fcc * fj.x * fk.y, gc = fab * fcd;
@@ -898,7 +947,7 @@ __global__ void __launch_bounds__(kBlk)
             double e = E[0];
 #pragma unroll
             for (int z = 1; z < NAL; ++z) e = q == z ? E[z] : e;
-            const double SQ = e * pv, SP = e * pd, SU = 2.0 * t.alpha[g][q] * SQ;
+            const double SQ = e * pv, SP = e * pd, SU = -2.0 * t.alpha[g][q] * SQ;
             const double c3 = fma(F, fma(-SP, iab, -SU), SQ * gc);
             const double c1 = fma(F, fma(SP, ca, -SU), SQ * ga) + c3;
             const double cc = fma(F, fma(SP, cb, -SU), SQ * gb) + c3;
@@ -993,6 +1042,14 @@ int split_of(int N) {
 
 namespace {
 
+// a = -alpha and 1024 a / ln 2 as an unevaluated sum (exp_fix)
+void exp_scale(double alpha, double *a, double *h, double *l) {
+  const DD v = dd_mul({-alpha, 0.0}, {0x1.71547652b82fep+10, 0x1.777d0ffda0d24p-46});
+  *a = -alpha;
+  *h = v.h;
+  *l = v.l;
+}
+
 // The table of a model, or false when its SF set keeps the generic kernels.
 bool w64_table(const SFDev &s, W64Tab *t) {
   *t = W64Tab{};
@@ -1005,13 +1062,13 @@ bool w64_table(const SFDev &s, W64Tab *t) {
   for (int q = 0; q < s.nrc; ++q) {
     t->rc[q] = s.rc_val[q];
     t->rc2[q] = s.rc_val[q] * s.rc_val[q];
-    fc_series(s.rc_val[q], &t->kv[q], t->fc.c[q]);
-    t->kd[q] = 2.0 * t->kv[q];  // fc'(r) / r = (d fc / dv) 2 kv
+    fc_series(s.rc_val[q], &t->kv[q], &t->fc.c[q]);
+    t->kd[q] = -t->kv[q];  // fc'(r) / r = (d fc / dw) kv
   }
   for (int q = 0; q < s.nrad; ++q) {
     t->rad_d[q] = s.rad_d[q];
     t->rad_rc[q] = s.rad_rc[q];
-    t->rad_alpha[q] = s.rad_alpha[q];
+    exp_scale(s.rad_alpha[q], &t->rad_a[q], &t->rad_ah[q], &t->rad_al[q]);
     t->rad_rs[q] = s.rad_rs[q];
   }
   int nal = 1, deg = 1;
@@ -1025,9 +1082,12 @@ bool w64_table(const SFDev &s, W64Tab *t) {
       deg = deg > s.ang_izeta[a] ? deg : s.ang_izeta[a];
       const double al = s.alpha_val[s.ang_alpha[a]];
       int q = 0;
-      while (q < n && t->alpha[g][q] != al) ++q;
+      while (q < n && t->alpha[g][q] != -al) ++q;
       if (q == 4) return false;
-      if (q == n) t->alpha[g][n++] = al;
+      if (q == n) {
+        exp_scale(al, &t->alpha[g][n], &t->alpha_h[g][n], &t->alpha_l[g][n]);
+        ++n;
+      }
       t->ang_d[a] = s.ang_d[a];
       t->ang_g[a] = g;
       t->ang_q[a] = q;
@@ -1057,13 +1117,8 @@ gapgb_status w64_prepare(gapgb_model *m) {
   if (m->d_w64 || m->w64_tried) return GAPGB_OK;
   m->w64_tried = true;
   if (!w64_table(m->sfh, &m->w64h)) return GAPGB_OK;
-  static const std::vector<double> T = [] {
-    std::vector<double> v(kExpN);
-    for (int j = 0; j < kExpN; ++j) v[j] = std::exp2((double)j / kExpN);
-    return v;
-  }();
-  GAPGB_CUDA_TRY(cudaMalloc(&m->d_exp64, sizeof(double) * kExpN));
-  GAPGB_CUDA_TRY(cudaMemcpy(m->d_exp64, T.data(), sizeof(double) * kExpN, cudaMemcpyHostToDevice));
+  GAPGB_CUDA_TRY(cudaMalloc(&m->d_exp64, 8 * kExpN));
+  GAPGB_CUDA_TRY(cudaMemcpy(m->d_exp64, exp2_table(), 8 * kExpN, cudaMemcpyHostToDevice));
   GAPGB_CUDA_TRY(cudaMalloc(&m->d_w64, sizeof(W64Tab)));
   GAPGB_CUDA_TRY(cudaMemcpy(m->d_w64, &m->w64h, sizeof(W64Tab), cudaMemcpyHostToDevice));
   return GAPGB_OK;
