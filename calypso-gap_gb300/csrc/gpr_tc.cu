@@ -17,17 +17,26 @@
 //                          wh.[mhT; mlT] (N = 128) and wl.mhT (N = 64)
 //   dE/dG_id = -(1/theta_d) (x''_id e_i - (W M'')_id)
 //
-// One CTA (8 warps) owns 128 atoms.  For each tile of 64 sparse points: one
-// 1-D bulk copy brings the pre-arranged operand tiles into shared memory,
-// one thread issues GEMM1 (8 tcgen05.mma, M=128 K=16, N=128 and N=64) into a
-// TMEM accumulator, the eight warps read it back with tcgen05.ld (thread =
-// atom row), form w, accumulate e and write wh/wl into shared memory as
-// GEMM2's A operand, and one thread issues GEMM2 (8 tcgen05.mma) accumulating
-// over all sparse tiles in a second TMEM region.  Fewer, wider MMAs: an
-// N = 128 MMA takes about 1.3 times as long as an N = 64 one on GB300, so the
-// 16 MMAs of a tile take about 0.76 times as long as 24 N = 64 MMAs.  The
-// [mh; ml] and [mhT; mlT] pairs are adjacent 64-row blocks in shared memory,
-// which is the 128-row B operand of the same canonical layout.
+// One CTA owns 128 atoms and walks the sparse points in tiles of 64.  Roles:
+// two sets of eight epilogue warps (thread = atom row and half of a tile's
+// columns) that take tiles in turn, a warp that issues GEMM1, one that issues
+// GEMM2, one that keeps a ring of five tiles loading.  C1 has three buffers of
+// 128 TMEM columns, so GEMM1 runs up to three tiles ahead; an epilogue warp
+// writes W (wh 16 + wl 16 columns) over the columns that it alone has read, and
+// GEMM2 takes W from there as its A operand.  C2 is the other 128 columns: one
+// CTA per SM.  Per SM an M = 128, K = 16 MMA takes 16 + N/2 cycles with A in
+// tensor memory and 48 + N/2 with A in shared memory (measured, N = 64 to 256),
+// so fewer, wider MMAs, and W in tensor memory: 760 + 500 cycles a tile.
+// Two warps issue because a warp's next barrier poll waits for the MMAs that it
+// has queued: with one, the pipe idles 350 cycles after each batch of eight.
+// Measured: a tile (128 atoms x 64 points) takes about 1650 cycles, 19 us x
+// M / 1000 for up to 152 x 128 atoms, 43 to 47 % of the tensor pipe's cycles
+// and 57 to 62 % of the issue slots; 19456 atoms, M = 4000: 61 us, where a
+// kernel of 4 warps per 128 atoms and two CTAs per SM, each with its GEMMs and
+// epilogue in turn and A and W in shared memory, took 131; 16384 atoms,
+// M = 8000: 108 us (241).  The [mh; ml] and [mhT; mlT] pairs are adjacent 64-row
+// blocks in shared memory, which is the 128-row B operand of the same canonical
+// layout.
 //
 // Operand tiles use the no-swizzle K-major canonical layout: 8-row x 16-byte
 // core matrices, K-adjacent cores 128 B apart (LBO), 8-row groups
@@ -53,35 +62,79 @@ constexpr int kTileK = 64;   // sparse points per tile (GEMM1 N, GEMM2 K)
 constexpr int kDP = 64;      // padded descriptor length (GEMM1 K, GEMM2 N)
 constexpr int kXBytes16 = kRows * kDP * 2;           // 128 x 64 bf16: 16 KB
 constexpr int kMBytes16 = kTileK * kDP * 2;          // 64 x 64 bf16: 8 KB
-constexpr int kWBytes = kRows * kTileK * 2;          // 128 x 64 bf16: 16 KB
 // per sparse tile image: mh, ml (64 x 64), mhT, mlT (64 x 64), b2[64], c[64]
 constexpr int kImgTile = 4 * kMBytes16 + 2 * kTileK * 4;     // 32.5 KB
 constexpr int kImgAtoms = 2 * kXBytes16;                      // xh, xl per 128 atoms
 
-// shared memory map (bytes from the 1024-aligned base); about 99 KB, so two
-// CTAs share an SM and one's GEMMs run under the other's epilogue
-constexpr int kOffXh = 0;
-constexpr int kOffXl = kOffXh + kXBytes16;
-constexpr int kOffImg = kOffXl + kXBytes16;              // one sparse tile image
-constexpr int kOffMh = kOffImg;
+// shared memory map (bytes from the 1024-aligned base): the ring of tile images
+constexpr int kStages = 5;
+constexpr int kStage = 33 * 1024;  // one tile image, padded
+constexpr int kOffMh = 0;
 constexpr int kOffMl = kOffMh + kMBytes16;
 constexpr int kOffMhT = kOffMl + kMBytes16;
 constexpr int kOffMlT = kOffMhT + kMBytes16;
+constexpr int kOffMnc = kOffMlT + kMBytes16;  // b2 and c
+static_assert(kImgTile <= kStage, "tile image beyond its stage");
 // [mh; ml] and [mhT; mlT] as one 128-row B operand: the second block starts
 // eight 8-row groups (the canonical layout's SBO apart) after the first
 static_assert(kOffMl - kOffMh == 8 * (kDP / 8) * 128, "mh / ml not one 128-row operand");
 static_assert(kOffMlT - kOffMhT == 8 * (kTileK / 8) * 128, "mhT / mlT not one 128-row operand");
-constexpr int kOffMnc = kOffMlT + kMBytes16;             // b2 and c, two tiles
-constexpr int kMncBytes = 2 * kTileK * 4;                 // one tile's mn and c
-constexpr int kOffWh = kOffMnc + 2 * kMncBytes;
-constexpr int kOffWl = kOffWh + kWBytes;
-constexpr int kOffBar = kOffWl + kWBytes;                 // 3 mbarriers + tmem base
-constexpr int kOffEp = kOffBar + 64;                      // partial energies [128] (FP64)
-constexpr int kSmemBytes = kOffEp + kRows * 8 + 1024;     // + alignment slack
-constexpr int kGprThreads = 256;  // warps w and w + 4 share TMEM lanes and split the columns
-constexpr int kTmemCols = 256;    // C1 and C2, two 64-column halves each
+constexpr int kOffX = kStages * kStage;                  // xh, xl
+constexpr int kOffBar = kOffX + kImgAtoms;
+constexpr int kOffEp = kOffBar + 512;                    // partial energies [128] (FP64)
+constexpr int kOffPart = kOffEp + kRows * 8;             // odd tiles' partial sums [3][256] float4
+constexpr int kSmemBytes = kOffPart + 3 * 2 * kRows * 16 + 1024;  // + alignment slack
+// two sets of 8 epilogue warps: w and w + 4 share TMEM lanes and split the columns
+constexpr int kEpiWarps = 16;
+constexpr int kGprThreads = 32 * (kEpiWarps + 3);  // and a warp each for GEMM1, GEMM2 and copies
+// TMEM columns
+constexpr int kC1 = 3;  // C1 / W buffers
+constexpr int kColC1 = 0, kColC2 = 128 * kC1;
 
-__global__ void __launch_bounds__(kGprThreads, 2)
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,"
+      "%14,%15,%16};" ::"r"(taddr),
+      "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
+      "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+      : "memory");
+}
+// v = (16 columns at taddr) + (16 columns at taddr + off), as tmem_ld32_sum2
+__device__ __forceinline__ void tmem_ld16_sum2(uint32_t taddr, uint32_t off, float (&v)[16]) {
+  uint32_t r[16], s[16];
+#define GAPGB_LD16(dst, addr)                                                                     \
+  asm volatile(                                                                                  \
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,"   \
+      "%14,%15}, [%16];"                                                                         \
+      : "=r"(dst[0]), "=r"(dst[1]), "=r"(dst[2]), "=r"(dst[3]), "=r"(dst[4]), "=r"(dst[5]),     \
+        "=r"(dst[6]), "=r"(dst[7]), "=r"(dst[8]), "=r"(dst[9]), "=r"(dst[10]), "=r"(dst[11]),   \
+        "=r"(dst[12]), "=r"(dst[13]), "=r"(dst[14]), "=r"(dst[15])                              \
+      : "r"(addr))
+  GAPGB_LD16(r, taddr);
+  GAPGB_LD16(s, taddr + off);
+#undef GAPGB_LD16
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+  for (int q = 0; q < 16; ++q) {
+    asm volatile("" : "+r"(r[q]), "+r"(s[q]));  // uses stay behind the wait
+    v[q] = __uint_as_float(r[q]) + __uint_as_float(s[q]);
+  }
+}
+// s += x with Kahan compensation c
+__device__ __forceinline__ void kahan(float &s, float &c, float x) {
+  const float y = x - c;
+  const float t = s + y;
+  c = (t - s) - y;
+  s = t;
+}
+__device__ __forceinline__ void tmem_st_wait() {
+  asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+
+__global__ void __launch_bounds__(kGprThreads, 1)
     k_gpr_tc(int N, int ntiles, const unsigned char *__restrict__ img_model,
              const unsigned char *__restrict__ img_atoms, const float *__restrict__ xs,
              const float *__restrict__ xn, const float *__restrict__ invth, int D,
@@ -90,25 +143,35 @@ __global__ void __launch_bounds__(kGprThreads, 2)
   unsigned char *sm = reinterpret_cast<unsigned char *>(
       ((uintptr_t)smraw + 1023) & ~(uintptr_t)1023);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int quad = warp & 3, half = warp >> 2;  // TMEM lane quadrant, column half
+  // epilogue warps: set, TMEM lane quadrant, column half
+  const int set = warp >> 3, quad = warp & 3, half = (warp >> 2) & 1;
   const uint32_t s_base = smem_u32(sm);
-  // bar_a: atoms (first tile), mh / ml and mn / c of a tile; bar_b: mhT / mlT
-  const uint32_t bar_a = s_base + kOffBar, bar_g1 = bar_a + 8, bar_g2 = bar_a + 16,
-                 bar_b = bar_a + 24;
-  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(sm + kOffBar + 32);
-  int *abort_flag = reinterpret_cast<int *>(sm + kOffBar + 40);
+  // a tile's image has arrived / is free (its GEMM2 done); C1 computed; W
+  // written; the atoms have arrived; given up; odd tiles' sums stored [3][8]
+  const uint32_t mfull = s_base + kOffBar, mempty = mfull + 8 * kStages,
+                 c1full = mempty + 8 * kStages, wfull = c1full + 8 * kC1, xfull = wfull + 8 * kC1,
+                 dead = xfull + 8, pfull = dead + 16;
+  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(sm + kOffBar + 384);
+  volatile int *abort_flag = reinterpret_cast<int *>(sm + kOffBar + 392);
   if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
-                     smem_u32(tmem_slot)),
-                 "n"(kTmemCols)
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(
+                     smem_u32(tmem_slot))
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   if (tid == 0) {
-    mbar_init(bar_a, 1);
-    mbar_init(bar_g1, 1);
-    mbar_init(bar_g2, 1);
-    mbar_init(bar_b, 1);
+    for (int q = 0; q < kStages; ++q) {
+      mbar_init(mfull + 8 * q, 1);
+      mbar_init(mempty + 8 * q, 1);
+    }
+    for (int q = 0; q < kC1; ++q) {
+      mbar_init(c1full + 8 * q, 1);
+      mbar_init(wfull + 8 * q, 8);
+    }
+    mbar_init(xfull, 1);
+    mbar_init(dead, 1);
+    mbar_init(dead + 8, 1);
+    for (int q = 0; q < 3 * 8; ++q) mbar_init(pfull + 8 * q, 1);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -116,195 +179,232 @@ __global__ void __launch_bounds__(kGprThreads, 2)
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *tmem_slot;
-  const uint32_t tC1 = tmem, tC2 = tmem + 2 * kTileK;
-  const uint32_t lane_base = (uint32_t)(quad * 32) << 16;  // this warp's TMEM lanes
-  const int row = quad * 32 + lane;                         // atom row of this thread
+  const uint32_t lane_base = tmem + ((uint32_t)(quad * 32) << 16);  // this warp's TMEM lanes
+  const int row = quad * 32 + lane;                                  // atom row of this thread
   const int i = blockIdx.x * kRows + row;
-  const float xnorm = (i < N) ? xn[i] : 0.f;
-  // w = c exp(-s/2) = c 2^(log2e v + a2_i + b2_k) with a2_i = -log2e |x''_i|^2 / 2
-  // and b2_k = -log2e |m''_k|^2 / 2 (the image stores b2): one add, one FMA
-  // and ex2 per element.  e = sum w: each thread sums its 32 elements of a
-  // tile into four plain partial sums (8 elements each), which enter four
-  // independent Kahan chains once per tile.
-  const float a2 = -0.5f * kLog2e * xnorm;
-  float esum[4] = {0.f, 0.f, 0.f, 0.f}, ecmp[4] = {0.f, 0.f, 0.f, 0.f};
-  // N = 128: [mh; ml] (GEMM1) or [mhT; mlT] (GEMM2); N = 64: mh or mhT alone
-  const uint32_t id_pair = instr_desc(kRows, 128), id1 = instr_desc(kRows, kTileK),
-                 id2 = instr_desc(kRows, kDP);
-  uint32_t ph_a = 0, ph_b = 0, ph_g1 = 0, ph_g2 = 0;
-  bool pend_a = false, pend_b = false, pend_g1 = false, pend_g2 = false;
   bool ok = true;
-  // two-stage copy pipeline: a tile's GEMM1 operands (mh, ml, mn, c) load
-  // while the previous tile's epilogue and GEMM2 run, its GEMM2 operands
-  // (mhT, mlT) while its own GEMM1 and epilogue run
-  auto load_a = [&](int t, bool first) {
-    if (tid == 0) {
-      const unsigned char *img = img_model + (size_t)t * kImgTile;
-      mbar_expect_tx(bar_a, 2 * kMBytes16 + kMncBytes + (first ? kImgAtoms : 0));
-      if (first)
-        bulk_g2s(s_base + kOffXh, img_atoms + (size_t)blockIdx.x * kImgAtoms, kImgAtoms, bar_a);
-      bulk_g2s(s_base + kOffMh, img, 2 * kMBytes16, bar_a);
-      bulk_g2s(s_base + kOffMnc + (t & 1) * kMncBytes, img + 4 * kMBytes16, kMncBytes, bar_a);
+  if (warp == kEpiWarps + 2) {
+    if (lane == 0) {
+      int t = 0;
+      mbar_expect_tx(xfull, kImgAtoms);
+      bulk_g2s(s_base + kOffX, img_atoms + (size_t)blockIdx.x * kImgAtoms, kImgAtoms, xfull);
+      for (; t < ntiles; ++t) {
+        const int q = t % kStages;
+        if (t >= kStages && !mbar_wait(mempty + 8 * q, (t / kStages - 1) & 1, flags)) break;
+        if (*abort_flag) break;
+        mbar_expect_tx(mfull + 8 * q, kImgTile);
+        bulk_g2s(s_base + q * kStage, img_model + (size_t)t * kImgTile, kImgTile, mfull + 8 * q);
+      }
+      if (t < ntiles) {
+        // gave up: one more bounded wait for each copy still in flight
+        *abort_flag = 1;
+        for (int u = t > kStages ? t - kStages : 0; u < t; ++u)
+          mbar_wait(mfull + 8 * (u % kStages), (u / kStages) & 1, flags);
+      }
+      mbar_wait(xfull, 0, flags);  // (also where there was no tile to use it)
     }
-    pend_a = true;
-  };
-  auto load_b = [&](int t) {
-    if (tid == 0) {
-      mbar_expect_tx(bar_b, 2 * kMBytes16);
-      bulk_g2s(s_base + kOffMhT, img_model + (size_t)t * kImgTile + 2 * kMBytes16,
-               2 * kMBytes16, bar_b);
-    }
-    pend_b = true;
-  };
-  if (ntiles > 0) {
-    load_a(0, true);
-    load_b(0);
-  }
-  for (int t = 0; t < ntiles && ok; ++t) {
-    const float *smn = reinterpret_cast<const float *>(sm + kOffMnc + (t & 1) * kMncBytes);
-    const float *sc = smn + kTileK;
-    ok = mbar_wait(bar_a, ph_a, flags);
-    if (ok) {
-      ph_a ^= 1;
-      pend_a = false;
-    }
-    if (!__syncthreads_and(ok)) break;
-    // GEMM1: C1[:, 0:64] + C1[:, 64:128] = xh.mh + xh.ml + xl.mh over K = 64
-    // (4 steps of 16): xh.[mh; ml] into both halves, then xl.mh into the first
-    if (tid == 0) {
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const uint32_t a_off[2] = {kOffXh, kOffXl};
-      for (int p = 0; p < 2; ++p)
-        for (int kk = 0; kk < kDP / 16; ++kk) {
-          const uint64_t ad = smem_desc(s_base + a_off[p] + kk * 256, 128, (kDP / 8) * 128);
-          const uint64_t bd = smem_desc(s_base + kOffMh + kk * 256, 128, (kDP / 8) * 128);
-          umma(tC1, ad, bd, p == 0 ? id_pair : id1, (p > 0 || kk > 0) ? 1u : 0u);
+  } else if (warp >= kEpiWarps) {
+    // N = 128: [mh; ml] (GEMM1) or [mhT; mlT] (GEMM2); N = 64: mh or mhT alone
+    const uint32_t id_pair = instr_desc(kRows, 128), id1 = instr_desc(kRows, kTileK);
+    auto wait = [&](uint32_t bar, uint32_t parity) {  // the warp as one
+      return __all_sync(0xffffffffu, mbar_wait(bar, parity, flags) && !*abort_flag) != 0;
+    };
+    int t = 0;
+    if (warp == kEpiWarps) {
+      // C1[:, 0:64] + C1[:, 64:128] = xh.mh + xh.ml + xl.mh over K = 64 (4 steps
+      // of 16): xh.[mh; ml] into both halves, then xl.mh into the first
+      const uint64_t da = smem_desc(s_base + kOffX, 128, (kDP / 8) * 128);
+      ok = ntiles > 0 && wait(xfull, 0);
+      for (; t < ntiles && ok; ++t) {
+        if (!(ok = wait(mfull + 8 * (t % kStages), (t / kStages) & 1))) break;
+        // W of tile t - 3 lies where C1 goes: its GEMM2 has to be done
+        const int u = t - kC1;
+        if (u >= 0 && !(ok = wait(mempty + 8 * (u % kStages), (u / kStages) & 1))) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t c1 = tmem + kColC1 + 128 * (t % kC1);
+        const uint64_t db =
+            smem_desc(s_base + (t % kStages) * kStage + kOffMh, 128, (kDP / 8) * 128);
+        if (elect_one()) {
+#pragma unroll
+          for (int p = 0; p < 2; ++p)
+#pragma unroll
+            for (int kk = 0; kk < kDP / 16; ++kk)
+              umma(c1, da + p * (kXBytes16 >> 4) + 16 * kk, db + 16 * kk, p == 0 ? id_pair : id1,
+                   (p > 0 || kk > 0) ? 1u : 0u);
+          umma_commit(c1full + 8 * (t % kC1));
         }
-      umma_commit(bar_g1);
+        __syncwarp();
+      }
+    } else {
+      // C2[:, 0:64] + C2[:, 64:128] += wh.mhT + wh.mlT + wl.mhT over K = 64
+      // (4 steps of 16): wh.[mhT; mlT] into both halves, wl.mhT into the first
+      for (; t < ntiles && ok; ++t) {
+        if (!(ok = wait(wfull + 8 * (t % kC1), (t / kC1) & 1))) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t w = tmem + kColC1 + 128 * (t % kC1);
+        const uint64_t db =
+            smem_desc(s_base + (t % kStages) * kStage + kOffMhT, 128, (kTileK / 8) * 128);
+        if (elect_one()) {
+#pragma unroll
+          for (int p = 0; p < 2; ++p)
+#pragma unroll
+            for (int kk = 0; kk < kTileK / 16; ++kk)
+              umma_ta(tmem + kColC2, w + 32 * (kk >> 1) + 16 * p + 8 * (kk & 1), db + 16 * kk,
+                      p == 0 ? id_pair : id1, (t > 0 || p > 0 || kk > 0) ? 1u : 0u);
+          umma_commit(mempty + 8 * (t % kStages));
+        }
+        __syncwarp();
+      }
     }
-    pend_g1 = true;
-    ok = mbar_wait(bar_g1, ph_g1, flags);
-    if (ok) {
-      ph_g1 ^= 1;
-      pend_g1 = false;
+    if (t < ntiles) {
+      // gave up: a last bounded wait for the MMAs issued so far
+      *abort_flag = 1;
+      const uint32_t bar = dead + 8 * (warp - kEpiWarps);
+      if (elect_one()) umma_commit(bar);
+      __syncwarp();
+      mbar_wait(bar, 0, flags);
     }
-    if (!__syncthreads_and(ok)) break;
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    // mh / ml are free again: the next tile's GEMM1 operands start loading
-    if (t + 1 < ntiles) load_a(t + 1, false);
-    // epilogue 1: w = c exp(-s/2), e += w, W tile (bf16 hi / lo) for GEMM2
-    unsigned char *wh = sm + kOffWh, *wl = sm + kOffWl;
-    constexpr int kHalfBlocks = kTileK / 64;  // 32-column blocks per column half
-#pragma unroll 1
-    for (int cc = kHalfBlocks * half; cc < kHalfBlocks * (half + 1); ++cc) {
-      float v[32];
-      tmem_ld32_sum2(tC1 + lane_base + cc * 32, kTileK, v);
+  } else {
+    const float xnorm = (i < N) ? xn[i] : 0.f;
+    // w = c exp(-s/2) = c 2^(log2e v + a2_i + b2_k) with a2_i = -log2e |x''_i|^2 / 2
+    // and b2_k = -log2e |m''_k|^2 / 2 (the image stores b2): one add, one FMA
+    // and ex2 per element.  The sets take tiles in turn, so that one computes
+    // while the other waits for TMEM.  e = sum w: each thread sums its 32
+    // elements of a tile into four plain partial sums (8 elements each), which
+    // enter four independent Kahan chains per (row, half) once per tile, in tile
+    // order.  Set 0 keeps the chains; set 1 hands it its sums through shared
+    // memory: three slots, since C1 of tile t + 6 waits for the W of tile t + 3,
+    // which set 0 writes after it has taken the sums of tile t.
+    const float a2 = -0.5f * kLog2e * xnorm;
+    float es[4] = {0.f, 0.f, 0.f, 0.f}, ec[4] = {0.f, 0.f, 0.f, 0.f};
+    float4 *slots = reinterpret_cast<float4 *>(sm + kOffPart) + half * kRows + row;
+    const uint32_t my_pfull = pfull + 8 * (warp & 7);
+    // the sums of odd tile t into set 0's chains
+    auto take = [&](int t) {
+      const int sl = (t >> 1) % 3;
+      if (!mbar_wait_w(my_pfull + 64 * sl, ((t >> 1) / 3) & 1, flags)) return false;
+      const float4 p = slots[sl * 2 * kRows];
+      kahan(es[0], ec[0], p.x);
+      kahan(es[1], ec[1], p.y);
+      kahan(es[2], ec[2], p.z);
+      kahan(es[3], ec[3], p.w);
+      return true;
+    };
+    for (int t = set; t < ntiles; t += 2) {
+      const int q = t % kStages;
+      ok = __all_sync(0xffffffffu, mbar_wait(mfull + 8 * q, (t / kStages) & 1, flags) &&
+                                       mbar_wait(c1full + 8 * (t % kC1), (t / kC1) & 1, flags) &&
+                                       !*abort_flag);
+      if (!ok) break;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const float *smn = reinterpret_cast<const float *>(sm + q * kStage + kOffMnc);
+      const float *sc = smn + kTileK;
+      const uint32_t c1 = lane_base + kColC1 + 128 * (t % kC1) + 32 * half;
       float part[4] = {0.f, 0.f, 0.f, 0.f};
+      uint32_t hpk[16], lpk[16];
 #pragma unroll
-      for (int g = 0; g < 4; ++g) {
-        uint32_t hpk[4], lpk[4];
-        const int kg = cc * 32 + g * 8;
-        const float4 b0 = *reinterpret_cast<const float4 *>(smn + kg);
-        const float4 b1 = *reinterpret_cast<const float4 *>(smn + kg + 4);
-        const float4 c0 = *reinterpret_cast<const float4 *>(sc + kg);
-        const float4 c1 = *reinterpret_cast<const float4 *>(sc + kg + 4);
-        const float bv[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
-        const float cv[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
+      for (int gg = 0; gg < 2; ++gg) {
+        float v[16];
+        tmem_ld16_sum2(c1 + 16 * gg, kTileK, v);
 #pragma unroll
-        for (int h = 0; h < 4; ++h) {
-          float w2[2];
+        for (int g = 2 * gg; g < 2 * gg + 2; ++g) {
+          const int kg = half * 32 + g * 8;
+          const float4 b0 = *reinterpret_cast<const float4 *>(smn + kg);
+          const float4 b1 = *reinterpret_cast<const float4 *>(smn + kg + 4);
+          const float4 f0 = *reinterpret_cast<const float4 *>(sc + kg);
+          const float4 f1 = *reinterpret_cast<const float4 *>(sc + kg + 4);
+          const float bv[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+          const float cv[8] = {f0.x, f0.y, f0.z, f0.w, f1.x, f1.y, f1.z, f1.w};
 #pragma unroll
-          for (int u = 0; u < 2; ++u) {
-            const int q = h * 2 + u;
-            const float w = cv[q] * ex2_approx(fmaf(v[g * 8 + q], kLog2e, a2 + bv[q]));
-            part[h] += w;
-            w2[u] = w;
+          for (int h = 0; h < 4; ++h) {
+            float w2[2];
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+              const int e = h * 2 + u;
+              const float w = cv[e] * ex2_approx(fmaf(v[(g & 1) * 8 + e], kLog2e, a2 + bv[e]));
+              part[h] += w;
+              w2[u] = w;
+            }
+            const __nv_bfloat162 hi = __floats2bfloat162_rn(w2[0], w2[1]);
+            const float2 hf = __bfloat1622float2(hi);
+            hpk[4 * g + h] = *reinterpret_cast<const uint32_t *>(&hi);
+            lpk[4 * g + h] = pack_bf16(w2[0] - hf.x, w2[1] - hf.y);
           }
-          const __nv_bfloat162 hi = __floats2bfloat162_rn(w2[0], w2[1]);
-          const float2 hf = __bfloat1622float2(hi);
-          hpk[h] = *reinterpret_cast<const uint32_t *>(&hi);
-          lpk[h] = pack_bf16(w2[0] - hf.x, w2[1] - hf.y);
         }
-        const int k0 = cc * 32 + g * 8;
-        const int off = kmajor_off(row, k0, kTileK / 8);
-        *reinterpret_cast<uint4 *>(wh + off) = make_uint4(hpk[0], hpk[1], hpk[2], hpk[3]);
-        *reinterpret_cast<uint4 *>(wl + off) = make_uint4(lpk[0], lpk[1], lpk[2], lpk[3]);
       }
+      // over the columns that this warp has just read: wh, wl of 32 points
+      tmem_st16(c1, hpk);
+      tmem_st16(c1 + 16, lpk);
+      tmem_st_wait();
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive(wfull + 8 * (t % kC1));
+      if (set == 1) {
+        const int sl = (t >> 1) % 3;
+        slots[sl * 2 * kRows] = make_float4(part[0], part[1], part[2], part[3]);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(my_pfull + 64 * sl);
+      } else {
+        if (t > 0 && !(ok = take(t - 1))) break;
 #pragma unroll
-      for (int h = 0; h < 4; ++h) {  // Kahan
-        const float y = part[h] - ecmp[h];
-        const float tt = esum[h] + y;
-        ecmp[h] = (tt - esum[h]) - y;
-        esum[h] = tt;
+        for (int h = 0; h < 4; ++h) kahan(es[h], ec[h], part[h]);
       }
     }
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    ok = mbar_wait(bar_b, ph_b, flags);
-    if (ok) {
-      ph_b ^= 1;
-      pend_b = false;
-    }
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    if (!__syncthreads_and(ok)) break;
-    // GEMM2: C2[:, 0:64] + C2[:, 64:128] += wh.mhT + wh.mlT + wl.mhT over
-    // K = 64 (4 steps of 16): wh.[mhT; mlT] into both halves, wl.mhT into the first
-    if (tid == 0) {
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const uint32_t a_off[2] = {kOffWh, kOffWl};
-      for (int p = 0; p < 2; ++p)
-        for (int kk = 0; kk < kTileK / 16; ++kk) {
-          const uint64_t ad = smem_desc(s_base + a_off[p] + kk * 256, 128, (kTileK / 8) * 128);
-          const uint64_t bd = smem_desc(s_base + kOffMhT + kk * 256, 128, (kTileK / 8) * 128);
-          umma(tC2, ad, bd, p == 0 ? id_pair : id2, (t > 0 || p > 0 || kk > 0) ? 1u : 0u);
-        }
-      umma_commit(bar_g2);
-    }
-    pend_g2 = true;
-    ok = mbar_wait(bar_g2, ph_g2, flags);  // operands are overwritten next tile
-    if (ok) {
-      ph_g2 ^= 1;
-      pend_g2 = false;
-    }
-    ok = __syncthreads_and(ok);
-    if (ok && t + 1 < ntiles) load_b(t + 1);
-  }
-  if (ok) {
+    if (set == 0 && ok && ntiles > 0 && (ntiles & 1) == 0) ok = take(ntiles - 1);
+    if (ok && ntiles > 0)
+      ok = __all_sync(0xffffffffu, mbar_wait(mempty + 8 * ((ntiles - 1) % kStages),
+                                             ((ntiles - 1) / kStages) & 1, flags));
+    if (!ok) *abort_flag = 1;
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     // the two column halves' partial energies, summed in a fixed order
     double *ep = reinterpret_cast<double *>(sm + kOffEp);
-    double emine = 0.0;
+    auto sync16 = [] { asm volatile("bar.sync 1, 512;" ::: "memory"); };  // the epilogue warps
+    double emine = (double)es[0] - (double)ec[0];
+    emine += (double)es[1] - (double)ec[1];
+    emine += (double)es[2] - (double)ec[2];
+    emine += (double)es[3] - (double)ec[3];
+    if (set == 0 && half == 1) ep[row] = emine;
+    sync16();
+    if (set == 0 && half == 0) ep[row] = emine + ep[row];
+    sync16();
+    if (!*abort_flag) {
+      // dE/dG: each thread a row and 16 components
+      const double etot = ep[row];
+      const int d0 = half * 32 + set * 16;
+      float c2[16];
+      tmem_ld16_sum2(lane_base + kColC2 + d0, kDP, c2);
+      if (i < N) {
+        if (set == 0 && half == 0) e_out[i] = etot;
+        const float ef = (float)etot;
+        float x[16];
 #pragma unroll
-    for (int h = 0; h < 4; ++h) emine += (double)esum[h] - (double)ecmp[h];
-    if (half == 1) ep[row] = emine;
-    __syncthreads();
-    if (half == 0) ep[row] = emine + ep[row];
-    __syncthreads();
-    const double etot = ep[row];
-    float c2[32];
-    tmem_ld32_sum2(tC2 + lane_base + half * 32, kDP, c2);
-    if (i < N) {
-      if (half == 0) e_out[i] = etot;
-      const float ef = (float)etot;
+        for (int k = 0; k < 16; k += 4)
+          *reinterpret_cast<float4 *>(x + k) =
+              *reinterpret_cast<const float4 *>(xs + (size_t)i * kDP + d0 + k);
+        float *o = dedg + (size_t)i * D + d0;
 #pragma unroll
-      for (int k = 0; k < 32; ++k) {
-        const int d = half * 32 + k;
-        if (d < D) dedg[(size_t)i * D + d] = -invth[d] * (xs[(size_t)i * kDP + d] * ef - c2[k]);
+        for (int k = 0; k < 16; ++k) {
+          const int d = d0 + k;
+          if (d < D) x[k] = -invth[d] * (x[k] * ef - c2[k]);
+        }
+        if (D % 4 == 0) {  // rows of dedg are then 16-byte aligned
+#pragma unroll
+          for (int k = 0; k < 16; k += 4)
+            if (d0 + k < D)
+              *reinterpret_cast<float4 *>(o + k) =
+                  make_float4(x[k], x[k + 1], x[k + 2], x[k + 3]);
+        } else {
+#pragma unroll
+          for (int k = 0; k < 16; ++k)
+            if (d0 + k < D) o[k] = x[k];
+        }
       }
     }
-  } else if (tid == 0) {
-    // a wait gave up: give the outstanding copy / MMA phases one more bounded
-    // wait before the tensor memory and shared memory are released
-    if (pend_a) mbar_wait(bar_a, ph_a, flags);
-    if (pend_b) mbar_wait(bar_b, ph_b, flags);
-    if (pend_g1) mbar_wait(bar_g1, ph_g1, flags);
-    if (pend_g2) mbar_wait(bar_g2, ph_g2, flags);
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   if (warp == 0)
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
-                 "n"(kTmemCols)
-                 : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
 }
 
 // x'' = G / theta - mu (FP32, row-padded to 64), |x''|^2, and the xh/xl tiles

@@ -87,6 +87,31 @@ __device__ __forceinline__ void umma_commit(uint32_t bar) {
       : "memory");
 }
 
+// D += A B with A in tensor memory (row = lane, two K values per column)
+__device__ __forceinline__ void umma_ta(uint32_t dtmem, uint32_t atmem, uint64_t bdesc,
+                                        uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+      " tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n" ::"r"(dtmem),
+      "r"(atmem), "l"(bdesc), "r"(idesc), "r"(accumulate));
+}
+
+// true in one lane of a warp in convergence.  A warp that issues MMAs runs its
+// loop and its waits as a whole and elects the lane only around the MMAs:
+// inside `if (lane == 0)` their operands sit in per-lane registers and each
+// MMA takes about 100 cycles to issue, longer than an N = 64 or 128 one runs.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t one;
+  asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n"
+               : "=r"(one));
+  return one != 0;
+}
+
+// bounded wait of a whole warp in convergence: the same answer for every lane
+__device__ __forceinline__ bool mbar_wait_w(uint32_t bar, uint32_t parity, int *flags) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, flags)) != 0;
+}
+
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float *v) {
   uint32_t r[32];
   asm volatile(
