@@ -223,21 +223,31 @@ struct W64Cut {
   unsigned long long c[kFcN];  // fc = sum (-1)^n c_n w^n, units of 2^-61
   unsigned long long ratio;    // r^2 to w: kv / 2 in units of 2^(-63 - E), rc^2 <= 2^E
   int top;                     // biased exponent of 2^(E - 1)
+  int up;                      // bits from the pairs' unit to the cutoff's own
+  unsigned long long rc2;      // rc^2 in the pairs' unit
 };
 struct W64Fc {
   W64Cut c[kMaxRC];
+  // fixed point: lengths below 2^(e - 1) in units of 2^(e - 64), their squares
+  // in units of 2^(2 e - 64) (e: pairs), radial arguments in 2^(er - 64)
+  int e, er;
+};
+struct W64Exp {  // exp(a x) of an x in fixed point: see exp_neg
+  double a;
+  unsigned long long m;
+  int frac, pad;
 };
 // 2^(j/1024) in units of 2^-63 (gpr64_tc.cu)
 constexpr int kExpN = 1024;
 const unsigned long long *exp2_table();
 struct W64Tab {
   int nsf, D, nrad, nang, nrc, ngrp, nal, deg;  // nal, deg: the kernels' template sizes
-  double rc[kMaxRC], rc2[kMaxRC], kv[kMaxRC], kd[kMaxRC];
+  double rc[kMaxRC], kv[kMaxRC], kd[kMaxRC];
   int rad_d[kMaxSF], rad_rc[kMaxSF];
-  // exponents as exp_fix takes them: a = -alpha and 1024 a / ln 2 in two parts
-  double rad_a[kMaxSF], rad_ah[kMaxSF], rad_al[kMaxSF], rad_rs[kMaxSF];
+  W64Exp rad_e[kMaxSF];  // a = -alpha
+  double rad_rs[kMaxSF];
   int grp_rc[kMaxRC], grp_start[kMaxRC + 1];
-  double alpha[kMaxRC][4], alpha_h[kMaxRC][4], alpha_l[kMaxRC][4];
+  W64Exp alpha[kMaxRC][4];
   int ang_d[kMaxSF], ang_g[kMaxSF], ang_q[kMaxSF];
   double bern[kMaxSF][5], mono[kMaxSF][5];
   W64Fc fc;  // the cutoffs' polynomials (also passed by value, for the constant bank)

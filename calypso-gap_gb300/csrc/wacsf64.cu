@@ -7,17 +7,18 @@
 // against 78.5 TFLOP/s), so these kernels are bound by the FP64 pipe and are
 // built to issue as few FP64 instructions as possible:
 //  - the pairs of slots within each angular cutoff are found in FP32 from the
-//    neighbour kernel's FP32 records (a conservative screen; the FP64 squared
+//    neighbour kernel's FP32 records (a conservative screen; the exact squared
 //    distance decides) and compacted into lists, so every lane of an FP64
 //    instruction works on a contributing pair;
 //  - fc(r) = (cos(pi r / rc) + 1) / 2 is an even, entire function of r: a
 //    polynomial of degree 11 in r^2, with fc'(r)/r from its derivative, so neither
 //    the slots nor the pairs take a cosine, and a pair takes no square root
 //    and no division either (every factor is written in r^2 and 1/r_slot);
-//  - that polynomial runs in 64-bit fixed point on the integer pipe, and so
-//    does the exponential past its argument reduction (a 1024-entry table of
-//    2^(j/1024) and a degree-4 polynomial): 5 FP64 instructions instead of 10,
-//    and 0 or 1 instead of 12 or 23, with errors below 0.5 and 1 ulp;
+//  - a pair's geometry (c^2, a^2 + b^2 + c^2, the dot product), that polynomial
+//    and the exponential (a 1024-entry table of 2^(j/1024) and a degree-4
+//    polynomial, argument reduction included) run in 64-bit fixed point on the
+//    integer pipe, where an instruction costs an SM sub-partition 1 to 2
+//    cycles, not 64; errors below 0.5 and 1 ulp;
 //  - the (1 +- cos)^zeta of a cutoff group are combinations of the products
 //    u^n w^(DEG-n) (u = (1 + cos)/2, w = 1 - u) with non-negative weights: a
 //    pair adds those products, times each alpha's exponential, to moments;
@@ -25,14 +26,14 @@
 //    so a pair needs one Horner pass for value and derivative, and it yields
 //    three scalars (s1 + s3, s2 + s3, s3); a slot's gradient is then
 //    d_q sum(s_own + s3) - sum(s3 d_other), gathered per slot.
-// Per pair of the standard set that is about 60 FP64 instructions for the
-// descriptors and 80 for the gradient, where the generic kernels issue about
+// Per pair of the standard set that is about 35 FP64 instructions for the
+// descriptors and 55 for the gradient, where the generic kernels issue about
 // 520 and 770.  Measured (ncu, both generic kernels -> these, split launches
-// included): 512 alloy atoms (56 slots, 690 pairs each) 520 -> 98 us and
-// 665 -> 161 us; 64 carbon atoms (158 slots, 7 cutoffs) 2380 -> 119 us and
-// 1858 -> 277 us; 6.2 k atoms of ragged cells 5444 -> 842 and 10177 -> 1330
-// us, of which the polynomial and the exponential on the integer pipe are the
-// last quarter (1139 and 1691 us with FP64 ones).
+// included): 512 alloy atoms (56 slots, 690 pairs each) 520 -> 82 us and
+// 665 -> 145 us; 64 carbon atoms (158 slots, 7 cutoffs) 2380 -> 102 us and
+// 1858 -> 259 us; 6.4 k atoms of ragged cells 5444 -> 604 and 10177 -> 1094
+// us (842 and 1330 with the geometry and the exponential's argument in FP64,
+// 1139 and 1691 with all of the polynomials there).
 //
 // A block of 4 warps works on one atom.  The pair list of each cutoff group
 // is cut into units of 512 pairs.  Small batches spread an atom's units over
@@ -57,6 +58,9 @@ constexpr int kClasses = 8;      // residue classes of units (bounds the split)
 
 typedef unsigned long long u64;
 typedef long long i64;
+struct __align__(32) I64x4 {
+  i64 x, y, z, w;
+};
 
 // x 2^sc as a double, rounded (0 < x < 2^63; otherwise zero)
 __device__ __forceinline__ double fix_double(u64 x, int sc) {
@@ -66,25 +70,45 @@ __device__ __forceinline__ double fix_double(u64 x, int sc) {
   return (i64)x > 0 ? __longlong_as_double((i64)b) : 0.0;
 }
 
-// w = r^2 / rc^2 (kv r^2 / 2) in units of 2^-64, below one
-__device__ __forceinline__ u64 fc_arg(double r2, const W64Cut &c) {
-  const u64 b = (u64)__double_as_longlong(r2);
-  const int sh = c.top - (int)(b >> 52);
+// x in units of 2^(E - 64), top = the biased exponent of 2^(E - 1) (x >= 0;
+// 2^E and more: the largest)
+__device__ __forceinline__ u64 to_fix(double x, int top) {
+  const u64 b = (u64)__double_as_longlong(x);
+  const int sh = top - (int)(b >> 52);
   const u64 m = ((b & 0xFFFFFFFFFFFFFull) | (1ull << 52)) << 11;
-  const u64 u = sh >= 64 ? 0 : (sh <= 0 ? m : m >> sh);
-  const u64 w = __umul64hi(u, c.ratio);
-  return (w >> 63) || sh < 0 ? ~0ull : w << 1;
+  return sh < 0 ? ~0ull : (sh >= 64 ? 0 : m >> sh);
+}
+__device__ __forceinline__ i64 to_fix_signed(double x, int top) {
+  const i64 m = (i64)to_fix(fabs(x), top);
+  return x < 0.0 ? -m : m;
+}
+__device__ __forceinline__ double signed_double(i64 x, int sc) {
+  const i64 sg = x >> 63;
+  return __longlong_as_double(__double_as_longlong(fix_double((u64)((x ^ sg) - sg), sc)) |
+                              (sg & (i64)(1ull << 63)));
+}
+
+// w = r^2 / rc^2 (kv r^2 / 2) in units of 2^-64, below one; r^2 in units of
+// 2^(E - 64), rc^2 <= 2^E
+__device__ __forceinline__ u64 fc_arg(u64 r2, const W64Cut &c) {
+  const u64 w = __umul64hi(r2, c.ratio);
+  return (w >> 63) ? ~0ull : w << 1;
+}
+__device__ __forceinline__ u64 slot_arg(double r2, const W64Cut &c) {
+  return fc_arg(to_fix(r2, c.top), c);
+}
+// of a pair within the cutoff: r^2 in the pairs' unit, `up` bits finer
+__device__ __forceinline__ u64 pair_arg(u64 r2, const W64Cut &c) {
+  return (r2 >> (64 - c.up)) ? ~0ull : fc_arg(r2 << c.up, c);
 }
 // fc = sum (-1)^n c_n w^n in integer arithmetic (units of 2^-61), and -d fc / dw
-__device__ __forceinline__ double fc_fix(const W64Cut &c, double r2) {
-  const u64 w = fc_arg(r2, c);
+__device__ __forceinline__ double fc_fix(const W64Cut &c, u64 w) {
   u64 p = c.c[kFcN - 1];
 #pragma unroll
   for (int n = kFcN - 2; n >= 0; --n) p = c.c[n] - __umul64hi(w, p);
   return fix_double(p, -61);
 }
-__device__ __forceinline__ void fc_fix2(const W64Cut &c, double r2, double &f, double &d) {
-  const u64 w = fc_arg(r2, c);
+__device__ __forceinline__ void fc_fix2(const W64Cut &c, u64 w, double &f, double &d) {
   u64 p = c.c[kFcN - 1], e = 0;
 #pragma unroll
   for (int n = kFcN - 2; n >= 0; --n) {
@@ -96,24 +120,24 @@ __device__ __forceinline__ void fc_fix2(const W64Cut &c, double r2, double &f, d
   d = (i64)e < 0 ? -fix_double(0ull - e, -61) : fix_double(e, -61);
 }
 
-// exp(a b), the product unrounded: 1024 a b / ln 2 = k + r with ah + al =
-// 1024 a / ln 2, then 2^(k/1024) from a table (P. T. P. Tang, "Table-driven
-// implementation of the exponential function in IEEE floating-point
-// arithmetic", ACM TOMS 15, 1989) and 2^(r/1024) by a degree-4 polynomial, in
-// integer arithmetic (exp2_fix of gpr64_tc.cu).  Outside the normal range, and
-// for NaN, the library's exp.
-__device__ __forceinline__ double exp_fix(double a, double ah, double al, double b,
+// exp(a v), a <= 0, of v = x 2^(e - 64): m x is |a| v 1024 / ln 2 with `frac`
+// fractional bits in its high word; its floor and fraction give 2^(k/1024) from
+// a table (P. T. P. Tang, "Table-driven implementation of the exponential
+// function in IEEE floating-point arithmetic", ACM TOMS 15, 1989) and
+// 2^(r/1024) by a degree-4 polynomial, all in integer arithmetic (exp2_fix of
+// gpr64_tc.cu).  The fraction is cut at 2^-50 (and 2^-50 off where it is zero):
+// a relative 2^-60.  Past the normal range, and for a > 0 (frac < 0), the
+// library's exp.
+__device__ __forceinline__ double exp_neg(const W64Exp &c, u64 x, int e,
                                           const u64 *__restrict__ T) {
-  const double kShift = 6755399441055744.0;  // 1.5 2^52: rounds to an integer in the low word
-  const double kf = fma(ah, b, kShift);
-  const double kd = kf - kShift;
-  if ((__double2hiint(kd) & 0x7fffffff) >= 0x412feb6c) return exp(a * b);  // |a b| >= 708
-  const double r = fma(al, b, fma(ah, b, -kd));  // within one of zero
-  const u64 f = (u64)__double_as_longlong(r + 6.0) & 0xFFFFFFFFFFFFFull;  // (r + 2) 2^50
-  const int k = __double2loint(kf) - 2 + (int)(f >> 50);
+  const u64 hi = __umul64hi(x, c.m), lo = x * c.m;
+  const u64 ki = hi >> (c.frac & 63);
+  if (c.frac < 0 || ki >= 1045929) return exp(c.a * fix_double(x >> 1, e - 63));  // |a v| >= 708
+  const u64 fr = c.frac >= 50 ? hi >> (c.frac - 50) : (hi << (50 - c.frac)) | (lo >> (14 + c.frac));
+  const int k = -1 - (int)ki;
   const u64 t = T[k & (kExpN - 1)];
   // y = the fraction of 1/1024 times ln 2, in units of 2^-74
-  const u64 y = __umul64hi((f & ((1ull << 50) - 1)) << 14, 0xB17217F7D1CF79ACull);
+  const u64 y = __umul64hi((~fr & ((1ull << 50) - 1)) << 14, 0xB17217F7D1CF79ACull);
   const u64 y2 = __umul64hi(y, y);                         // 2^-84
   const uint32_t yh = (uint32_t)(y >> 32);                 // 2^-42
   const uint32_t y3 = __umulhi((uint32_t)(y2 >> 32), yh);  // 2^-62
@@ -161,7 +185,7 @@ __device__ __forceinline__ void warp_fold(double (&v)[N], int lane, double *out,
 
 // shared-memory layout (bytes), common to the kernels
 struct Lay {
-  size_t A, B, R, fc, f4, idx, mask, pre, row, list, rest, total;
+  size_t A, B, I, fc, f4, idx, mask, pre, row, list, rest, total;
 };
 __host__ __device__ inline size_t up32(size_t x) { return (x + 31) / 32 * 32; }
 __host__ __device__ inline Lay layout(int capS, int nrc, size_t rest) {
@@ -169,11 +193,11 @@ __host__ __device__ inline Lay layout(int capS, int nrc, size_t rest) {
   const size_t c = capS;
   Lay l;
   size_t o = kExpN * 8;
-  l.A = o, o += c * 32;                  // dx, dy, dz, r^2/2
+  l.A = o, o += c * 32;                  // dx, dy, dz, r
+  l.I = o, o += c * 32;                  // dx, dy, dz, r^2/2 in fixed point
   l.B = o, o += up32(c * 16);            // 1/r, weight
   l.fc = o, o += up32(c * nrc * 16);     // fc, fc'/r of every cutoff
   l.f4 = o, o += up32(c * 16);           // FP32 dx, dy, dz, r
-  l.R = o, o += up32(c * 8);             // r
   l.idx = o, o += up32(c * 2);           // the group's slots (those within its cutoff)
   l.mask = o, o += up32(c * W * 4);      // pair bits of the group's slots, a row's words adjacent
   l.pre = o, o += up32(c * W * 2);       // the row's pairs k > j before each word
@@ -188,7 +212,7 @@ struct View {
   const u64 *T;
   double4 *A;
   double2 *B, *fc;
-  double *R;
+  I64x4 *I;
   float4 *f4;
   unsigned *mask;
   unsigned short *idx, *pre;
@@ -201,7 +225,7 @@ __device__ __forceinline__ View view(unsigned char *sm, const Lay &l) {
   v.A = reinterpret_cast<double4 *>(sm + l.A);
   v.B = reinterpret_cast<double2 *>(sm + l.B);
   v.fc = reinterpret_cast<double2 *>(sm + l.fc);
-  v.R = reinterpret_cast<double *>(sm + l.R);
+  v.I = reinterpret_cast<I64x4 *>(sm + l.I);
   v.f4 = reinterpret_cast<float4 *>(sm + l.f4);
   v.idx = reinterpret_cast<unsigned short *>(sm + l.idx);
   v.mask = reinterpret_cast<unsigned *>(sm + l.mask);
@@ -224,19 +248,24 @@ __device__ __forceinline__ int stage(const View &s, const W64Tab &t, const W64Fc
     const size_t g = (size_t)i * cap + q;
     const double4 e = xyzr[g];
     const double r = e.w;
-    s.A[q] = make_double4(e.x - pi.x, e.y - pi.y, e.z - pi.z, 0.5 * (r * r));
+    const double dx = e.x - pi.x, dy = e.y - pi.y, dz = e.z - pi.z;
+    s.A[q] = make_double4(dx, dy, dz, r);
     s.f4[q] = d32[g];
     if (!want_fc) continue;
-    s.R[q] = r;
+    const int top = fc.e - 1 + 1023;
+    I64x4 v;
+    v.x = to_fix_signed(dx, top), v.y = to_fix_signed(dy, top), v.z = to_fix_signed(dz, top);
+    v.w = (i64)to_fix(0.5 * (r * r), 2 * fc.e - 1 + 1023);
+    s.I[q] = v;
     s.B[q] = make_double2(1.0 / r, apos[nj[g]].w);
     for (int c = 0; c < t.nrc; ++c) {
       double f = 0.0, d = 0.0;
       if (r <= t.rc[c]) {
         if (GRAD) {
-          fc_fix2(fc.c[c], r * r, f, d);
+          fc_fix2(fc.c[c], slot_arg(r * r, fc.c[c]), f, d);
           d *= t.kd[c];
         } else {
-          f = fc_fix(fc.c[c], r * r);
+          f = fc_fix(fc.c[c], slot_arg(r * r, fc.c[c]));
         }
       }
       s.fc[(size_t)c * capS + q] = make_double2(f, d);
@@ -316,6 +345,29 @@ __device__ __forceinline__ unsigned upper(const View &s, int W, int j, int w) {
   return w > (j >> 5) ? m : (w < (j >> 5) ? 0u : m & ~((2u << (j & 31)) - 1u));
 }
 
+// A pair of slots in fixed point: c^2 and a^2 + b^2 + c^2 (units of 2^(2 e - 64)),
+// and (a^2 + b^2 - c^2) / 2.  The differences are below the cutoff, 2^(e - 1),
+// whatever wraps before.  Integer instructions, two FP64 ones less per
+// coordinate; the unit is finer than an FP64 square's last place from 0.1 A up.
+struct Pair {
+  u64 c2, s3;
+  i64 dot;
+};
+__device__ __forceinline__ Pair pair_of(const View &s, int j, int k) {
+  const I64x4 a = s.I[j], b = s.I[k];
+  auto sq = [](i64 d) {
+    const u64 m = (u64)(d < 0 ? -d : d);
+    return __umul64hi(m, m);
+  };
+  Pair p;
+  p.c2 = sq((i64)((u64)a.x - (u64)b.x)) + sq((i64)((u64)a.y - (u64)b.y)) +
+         sq((i64)((u64)a.z - (u64)b.z));
+  const u64 h = (u64)a.w + (u64)b.w;
+  p.s3 = 2 * h + p.c2;
+  p.dot = (i64)(h - (p.c2 >> 1));
+  return p;
+}
+
 // list[p - p0] = j | k << 16 (slots) for the pairs p in [p0, p1).  Ends with a
 // barrier.
 __device__ __forceinline__ void expand(const View &s, int n, int p0, int p1) {
@@ -372,11 +424,12 @@ __global__ void __launch_bounds__(kBlk, NAL * (DEG + 1) <= 10 ? 5 : 3)
       const int ng = kBlk / t.nrad, sr = tid % t.nrad, gr = tid / t.nrad;
       double acc = 0.0, accw = 0.0;
       if (gr < ng) {
-        const double al = t.rad_a[sr], ah = t.rad_ah[sr], alo = t.rad_al[sr], rs = t.rad_rs[sr];
+        const W64Exp ex = t.rad_e[sr];
+        const double rs = t.rad_rs[sr];
         const double2 *f = s.fc + (size_t)t.rad_rc[sr] * capS;
         for (int q = gr; q < P; q += ng) {
-          const double fq = f[q].x, u = s.R[q] - rs;
-          const double e = exp_fix(al, ah, alo, u * u, s.T);
+          const double fq = f[q].x, u = s.A[q].w - rs;
+          const double e = exp_neg(ex, to_fix(u * u, fc.er - 1 + 1023), fc.er, s.T);
           const double v = __double2hiint(fq) != 0 ? e * fq : 0.0;  // beyond the cutoff: zero
           acc += v;
           accw = fma(v, s.B[q].y, accw);
@@ -401,15 +454,10 @@ __global__ void __launch_bounds__(kBlk, NAL * (DEG + 1) <= 10 ? 5 : 3)
       int n;
       const int np = build_pairs<false>(s, t, g, P, n);
       const int rci = t.grp_rc[g];
-      const i64 rc2 = __double_as_longlong(t.rc2[rci]);
       const double2 *f = s.fc + (size_t)rci * capS;
-      double al[NAL], ah[NAL], alo[NAL];
+      W64Exp ex[NAL];
 #pragma unroll
-      for (int q = 0; q < NAL; ++q) {
-        al[q] = t.alpha[g][q];
-        ah[q] = t.alpha_h[g][q];
-        alo[q] = t.alpha_l[g][q];
-      }
+      for (int q = 0; q < NAL; ++q) ex[q] = t.alpha[g][q];
       const int nu = (np + kUnit - 1) / kUnit;
       for (int u = 0; u < nu; ++u) {
         const int cls = (u0 + u) % kClasses;
@@ -423,17 +471,13 @@ __global__ void __launch_bounds__(kBlk, NAL * (DEG + 1) <= 10 ? 5 : 3)
           const bool live = p < p1;
           const unsigned jk = live ? s.list[p - p0] : 0u;
           const int j = jk & 0xffff, k = jk >> 16;
-          const double4 aj = s.A[j], ak = s.A[k];
-          const double cx = aj.x - ak.x, cy = aj.y - ak.y, cz = aj.z - ak.z;
-          const double c2 = fma(cx, cx, fma(cy, cy, cz * cz));
+          const Pair pr = pair_of(s, j, k);
           const double2 bj = s.B[j], bk = s.B[k];
-          double fcc = fc_fix(fc.c[rci], c2);
-          const bool in = live && __double_as_longlong(c2) <= rc2;  // else exactly zero
+          double fcc = fc_fix(fc.c[rci], pair_arg(pr.c2, fc.c[rci]));
+          const bool in = live && pr.c2 <= fc.c[rci].rc2;  // else exactly zero
           fcc = in ? fcc : 0.0;
           // costheta = (rij^2 + rik^2 - rjk^2) / (2 rij rik) (wacsf.f90:271-273)
-          const double sab = aj.w + ak.w;
-          const double cosv = fma(-0.5, c2, sab) * (bj.x * bk.x);
-          const double s3 = fma(2.0, sab, c2);
+          const double cosv = signed_double(pr.dot, 2 * fc.e - 64) * (bj.x * bk.x);
           const double F = f[j].x * f[k].x * fcc;
           const double wjk = bj.y * bk.y;
           const double uu = fma(0.5, cosv, 0.5), ww = fma(-0.5, cosv, 0.5);
@@ -455,7 +499,7 @@ __global__ void __launch_bounds__(kBlk, NAL * (DEG + 1) <= 10 ? 5 : 3)
           }
 #pragma unroll
           for (int q = 0; q < NAL; ++q) {
-            const double ef = in ? exp_fix(al[q], ah[q], alo[q], s3, s.T) * F : 0.0;
+            const double ef = in ? exp_neg(ex[q], pr.s3, 2 * fc.e, s.T) * F : 0.0;
             const double efw = ef * wjk;
 #pragma unroll
             for (int n = 0; n < NB; ++n) {
@@ -645,20 +689,20 @@ __global__ void __launch_bounds__(kBlk, 4)
     // (exp fc)'/r = exp (-2 alpha (1 - rs/r) fc + fc'/r)
     if (y == split - 1)
       for (int q = tid; q < P; q += kBlk) {
-        const double r = s.R[q], r2 = 2.0 * s.A[q].w;
+        const double r = s.A[q].w, r2 = r * r;
         const double2 b = s.B[q];
         double sum = 0.0;
         for (int a = 0; a < t.nrad; ++a) {
           const double2 f = s.fc[(size_t)t.rad_rc[a] * capS + q];
           if ((__double2hiint(f.x) | __double2hiint(f.y)) == 0) continue;  // beyond the cutoff
-          const double al = t.rad_a[a], rs = t.rad_rs[a];
+          const double al = t.rad_e[a].a, rs = t.rad_rs[a];
           double u2 = r2, ur = 1.0;
           if (rs != 0.0) {  // uniform over the block
             const double u = r - rs;
             u2 = u * u;
             ur = u * b.x;
           }
-          const double e = exp_fix(al, t.rad_ah[a], t.rad_al[a], u2, s.T);
+          const double e = exp_neg(t.rad_e[a], to_fix(u2, fc.er - 1 + 1023), fc.er, s.T);
           const double g = fma(2.0 * al * ur, f.x, f.y);
           sum = fma(fma(dg[t.rad_d[a] + t.nsf], b.y, dg[t.rad_d[a]]) * e, g, sum);
         }
@@ -672,7 +716,6 @@ __global__ void __launch_bounds__(kBlk, 4)
       const int np = build_pairs<true>(s, t, g, P, n);
       const int rci = t.grp_rc[g];
       const double kd = t.kd[rci];
-      const i64 rc2 = __double_as_longlong(t.rc2[rci]);
       const double2 *f = s.fc + (size_t)rci * capS;
       // dE/dG contracted onto polynomials in cos: cell (weighting, alpha, power)
       for (int c = tid; c < 2 * NAL * NB; c += kBlk) {
@@ -682,13 +725,9 @@ __global__ void __launch_bounds__(kBlk, 4)
           if (t.ang_q[a] == q) v = fma(t.mono[a][m], dg[t.ang_d[a] + (h ? t.nsf : 0)], v);
         sU[c] = v;
       }
-      double al[NAL], ah[NAL], alo[NAL];
+      W64Exp ex[NAL];
 #pragma unroll
-      for (int q = 0; q < NAL; ++q) {
-        al[q] = t.alpha[g][q];
-        ah[q] = t.alpha_h[g][q];
-        alo[q] = t.alpha_l[g][q];
-      }
+      for (int q = 0; q < NAL; ++q) ex[q] = t.alpha[g][q];
       __syncthreads();
       double4 *sc = split > 1 ? scr + (size_t)i * nsc + (size_t)u0 * kUnit
                               : scr + (size_t)blockIdx.x * nsc;
@@ -702,25 +741,21 @@ __global__ void __launch_bounds__(kBlk, 4)
           const bool live = p < p1;
           const unsigned jk = live ? s.list[p - p0] : 0u;
           const int j = jk & 0xffff, k = jk >> 16;
-          const double4 aj = s.A[j], ak = s.A[k];
-          const double cx = aj.x - ak.x, cy = aj.y - ak.y, cz = aj.z - ak.z;
-          const double c2 = fma(cx, cx, fma(cy, cy, cz * cz));
+          const Pair pr = pair_of(s, j, k);
           const double2 bj = s.B[j], bk = s.B[k], fj = f[j], fk = f[k];
           double fcc, fcd;
-          fc_fix2(fc.c[rci], c2, fcc, fcd);
+          fc_fix2(fc.c[rci], pair_arg(pr.c2, fc.c[rci]), fcc, fcd);
           fcd *= kd;
-          const bool in = live && __double_as_longlong(c2) <= rc2;
+          const bool in = live && pr.c2 <= fc.c[rci].rc2;
           fcc = in ? fcc : 0.0;
           fcd = in ? fcd : 0.0;
           const double iab = bj.x * bk.x;
-          const double sab = aj.w + ak.w;
-          const double cosv = fma(-0.5, c2, sab) * iab;
-          const double s3 = fma(2.0, sab, c2);
+          const double cosv = signed_double(pr.dot, 2 * fc.e - 64) * iab;
           const double wjk = bj.y * bk.y;
           double SP = 0.0, SQ = 0.0, SU = 0.0;
 #pragma unroll
           for (int q = 0; q < NAL; ++q) {
-            const double e = in ? exp_fix(al[q], ah[q], alo[q], s3, s.T) : 0.0;
+            const double e = in ? exp_neg(ex[q], pr.s3, 2 * fc.e, s.T) : 0.0;
             const double *U0 = sU + q * NB, *U1 = sU + (NAL + q) * NB;
             double pv = fma(wjk, U1[DEG], U0[DEG]), pd = 0.0;
 #pragma unroll
@@ -730,7 +765,7 @@ __global__ void __launch_bounds__(kBlk, 4)
             }
             const double x = e * pv;
             SQ += x;
-            SU = fma(-2.0 * al[q], x, SU);
+            SU = fma(-2.0 * ex[q].a, x, SU);
             SP = fma(e, pd, SP);
           }
           // d/da of [P(cos) E fc(a) fc(b) fc(c)], over a; likewise b and c:
@@ -889,8 +924,8 @@ __global__ void __launch_bounds__(kBlk)
       const double2 f = s.fc[(size_t)t.rad_rc[a] * capS + q], b = s.B[q];
       if ((__double2hiint(f.x) | __double2hiint(f.y)) == 0) continue;  // beyond the cutoff
       const double4 d = s.A[q];
-      const double al = t.rad_a[a], u = s.R[q] - t.rad_rs[a];
-      const double v = exp_fix(al, t.rad_ah[a], t.rad_al[a], u * u, s.T) *
+      const double al = t.rad_e[a].a, u = d.w - t.rad_rs[a];
+      const double v = exp_neg(t.rad_e[a], to_fix(u * u, fc.er - 1 + 1023), fc.er, s.T) *
                        fma(2.0 * al * (u * b.x), f.x, f.y);
       const double dd[3] = {d.x, d.y, d.z};
 #pragma unroll
@@ -906,7 +941,6 @@ __global__ void __launch_bounds__(kBlk)
       const int np = build_pairs<true>(s, t, g, P, n);
       const int rci = t.grp_rc[g], s0 = t.grp_start[g], na = t.grp_start[g + 1] - s0;
       const double kd = t.kd[rci];
-      const i64 rc2 = __double_as_longlong(t.rc2[rci]);
       const double2 *f = s.fc + (size_t)rci * capS;
       double4 *sc = scr + (size_t)blockIdx.x * nsc;
       for (int p0 = 0; p0 < np; p0 += kUnit) {
@@ -917,21 +951,19 @@ __global__ void __launch_bounds__(kBlk)
           if (p >= p1) continue;
           const unsigned jk = s.list[p - p0];
           const int j = jk & 0xffff, k = jk >> 16;
-          const double4 aj = s.A[j], ak = s.A[k];
-          const double cx = aj.x - ak.x, cy = aj.y - ak.y, cz = aj.z - ak.z;
-          const double c2 = fma(cx, cx, fma(cy, cy, cz * cz));
+          const Pair pr = pair_of(s, j, k);
           const double2 bj = s.B[j], bk = s.B[k], fj = f[j], fk = f[k];
           double fcc, fcd;
-          fc_fix2(fc.c[rci], c2, fcc, fcd);
-          const bool in = __double_as_longlong(c2) <= rc2;
+          fc_fix2(fc.c[rci], pair_arg(pr.c2, fc.c[rci]), fcc, fcd);
+          const bool in = pr.c2 <= fc.c[rci].rc2;
           fcc = in ? fcc : 0.0;
           fcd = in ? fcd * kd : 0.0;
-          const double iab = bj.x * bk.x, sab = aj.w + ak.w;
-          const double cosv = fma(-0.5, c2, sab) * iab, s3 = fma(2.0, sab, c2);
+          const double iab = bj.x * bk.x;
+          const double cosv = signed_double(pr.dot, 2 * fc.e - 64) * iab;
           double E[NAL];
 #pragma unroll
           for (int q = 0; q < NAL; ++q)
-            E[q] = in ? exp_fix(t.alpha[g][q], t.alpha_h[g][q], t.alpha_l[g][q], s3, s.T) : 0.0;
+            E[q] = in ? exp_neg(t.alpha[g][q], pr.s3, 2 * fc.e, s.T) : 0.0;
           const double fab = fj.x * fk.x, F = fab * fcc;
           const double ca = fma(-cosv, bj.x * bj.x, iab), cb = fma(-cosv, bk.x * bk.x, iab);
           const double ga = fcc * fk.x * fj.y, gb = fcc * fj.x * fk.y, gc = fab * fcd;
@@ -947,7 +979,7 @@ __global__ void __launch_bounds__(kBlk)
             double e = E[0];
 #pragma unroll
             for (int z = 1; z < NAL; ++z) e = q == z ? E[z] : e;
-            const double SQ = e * pv, SP = e * pd, SU = -2.0 * t.alpha[g][q] * SQ;
+            const double SQ = e * pv, SP = e * pd, SU = -2.0 * t.alpha[g][q].a * SQ;
             const double c3 = fma(F, fma(-SP, iab, -SU), SQ * gc);
             const double c1 = fma(F, fma(SP, ca, -SU), SQ * ga) + c3;
             const double cc = fma(F, fma(SP, cb, -SU), SQ * gb) + c3;
@@ -1042,12 +1074,23 @@ int split_of(int N) {
 
 namespace {
 
-// a = -alpha and 1024 a / ln 2 as an unevaluated sum (exp_fix)
-void exp_scale(double alpha, double *a, double *h, double *l) {
-  const DD v = dd_mul({-alpha, 0.0}, {0x1.71547652b82fep+10, 0x1.777d0ffda0d24p-46});
-  *a = -alpha;
-  *h = v.h;
-  *l = v.l;
+// e = -alpha as exp_neg takes it, for arguments in units of 2^(E - 64)
+W64Exp exp_scale(double alpha, int E) {
+  W64Exp c = {-alpha, 0, 50, 0};
+  if (alpha == 0.0) return c;
+  const DD v = dd_mul({alpha, 0.0}, {0x1.71547652b82fep+10, 0x1.777d0ffda0d24p-46});
+  int ea;
+  std::frexp(v.h, &ea);
+  c.frac = 64 - E - ea;
+  if (!(alpha > 0.0 && std::isfinite(v.h)) || c.frac <= 0) {
+    c.frac = -1;
+    return c;
+  }
+  c.frac = std::min(c.frac, 63);
+  const int bits = c.frac + E;  // m = 1024 alpha / ln 2 2^bits
+  c.m = (unsigned long long)((__int128)std::ldexp(v.h, bits) +
+                             (__int128)std::llround(std::ldexp(v.l, bits)));
+  return c;
 }
 
 // The table of a model, or false when its SF set keeps the generic kernels.
@@ -1059,16 +1102,30 @@ bool w64_table(const SFDev &s, W64Tab *t) {
   t->nang = s.nang;
   t->nrc = s.nrc;
   t->ngrp = s.n_ang_grp;
+  // the fixed-point units: 2^(e - 1) above every cutoff (with the screen's
+  // margin), 2^er above every (r - rs)^2 within its cutoff
+  double rmax = 0.0, u2max = 0.0;
+  for (int q = 0; q < s.nrc; ++q) rmax = std::max(rmax, s.rc_val[q]);
+  for (int q = 0; q < s.nrad; ++q) {
+    const double u = std::max(std::fabs(s.rad_rs[q]), std::fabs(s.rc_val[s.rad_rc[q]] - s.rad_rs[q]));
+    u2max = std::max(u2max, u * u);
+  }
+  std::frexp(1.001 * rmax, &t->fc.e);
+  t->fc.e += 1;
+  std::frexp(std::max(u2max, 1e-30) * 1.001, &t->fc.er);
   for (int q = 0; q < s.nrc; ++q) {
     t->rc[q] = s.rc_val[q];
-    t->rc2[q] = s.rc_val[q] * s.rc_val[q];
     fc_series(s.rc_val[q], &t->kv[q], &t->fc.c[q]);
+    // (a cutoff 2^30 times shorter than the longest: left to the generic kernels)
+    t->fc.c[q].up = 2 * t->fc.e - (t->fc.c[q].top - 1022);
+    if (t->fc.c[q].up > 62) return false;
+    t->fc.c[q].rc2 = (unsigned long long)std::ldexp(s.rc_val[q] * s.rc_val[q], 64 - 2 * t->fc.e);
     t->kd[q] = -t->kv[q];  // fc'(r) / r = (d fc / dw) kv
   }
   for (int q = 0; q < s.nrad; ++q) {
     t->rad_d[q] = s.rad_d[q];
     t->rad_rc[q] = s.rad_rc[q];
-    exp_scale(s.rad_alpha[q], &t->rad_a[q], &t->rad_ah[q], &t->rad_al[q]);
+    t->rad_e[q] = exp_scale(s.rad_alpha[q], t->fc.er);
     t->rad_rs[q] = s.rad_rs[q];
   }
   int nal = 1, deg = 1;
@@ -1082,11 +1139,10 @@ bool w64_table(const SFDev &s, W64Tab *t) {
       deg = deg > s.ang_izeta[a] ? deg : s.ang_izeta[a];
       const double al = s.alpha_val[s.ang_alpha[a]];
       int q = 0;
-      while (q < n && t->alpha[g][q] != -al) ++q;
+      while (q < n && t->alpha[g][q].a != -al) ++q;
       if (q == 4) return false;
       if (q == n) {
-        exp_scale(al, &t->alpha[g][n], &t->alpha_h[g][n], &t->alpha_l[g][n]);
-        ++n;
+        t->alpha[g][n++] = exp_scale(al, 2 * t->fc.e);
       }
       t->ang_d[a] = s.ang_d[a];
       t->ang_g[a] = g;
