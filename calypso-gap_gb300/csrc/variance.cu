@@ -179,7 +179,7 @@ constexpr int kVOffBar = kVStages * kVStage;
 constexpr int kVOffEp = kVOffBar + 128;     // partial dots of the second column half
 constexpr int kVSmem = kVOffEp + kVRows * 8 + 1024;
 constexpr int kVThreads = 256;
-constexpr int kKimgDC = 32;                 // descriptor chunk of the K-image kernel
+constexpr int kKimgDC = 64;                 // descriptor components of the K-image kernel's tiles
 
 // K image: block (atom tile a, chunk c) = 128 rows x 32 sparse points, hi
 // then lo, no-swizzle K-major (k = sparse point index within the chunk)
@@ -197,66 +197,75 @@ __global__ void k_var_center(int row0, int rows, int D, const TG *__restrict__ G
   xc[e] = (float)((double)G[(size_t)row0 * D + e] * invth[d] - mu[d]);
 }
 
+// A subtraction and an FMA per atom, point and component, whose order is kept:
+// 54 % of the FP32 rate.  A block takes `per` chunks of points and, up to 64
+// components, stages its 128 atoms once for all of them: 419 us at 16384 atoms,
+// 4000 points, 443 with one chunk per block and components padded to 32.  Four
+// atoms per thread instead of two (fewer shared-memory loads per FMA, fewer
+// warps) took 30 us longer.
 __global__ void __launch_bounds__(256)
-    k_var_kimg(int rows, int M, int D, int nch, const float *__restrict__ xc,
+    k_var_kimg(int rows, int M, int D, int nch, int per, const float *__restrict__ xc,
                const float *__restrict__ mc, unsigned char *__restrict__ img) {
   __shared__ __align__(16) float xs[kKimgDC][kVRows + 4];
   __shared__ __align__(16) float ms[kKimgDC][kVK + 4];
   const int tid = threadIdx.x;
-  const int c = blockIdx.x, a = blockIdx.y;
+  const int a = blockIdx.y, c0 = blockIdx.x * per, c1 = min(nch, c0 + per);
   const int r0 = (tid >> 2) * 2, k0 = (tid & 3) * 8;
-  float acc[2][8];
+  for (int c = c0; c < c1; ++c) {
+    float acc[2][8];
 #pragma unroll
-  for (int q = 0; q < 2; ++q)
+    for (int q = 0; q < 2; ++q)
 #pragma unroll
-    for (int u = 0; u < 8; ++u) acc[q][u] = 0.f;
-  for (int d0 = 0; d0 < D; d0 += kKimgDC) {
-    for (int e = tid; e < kVRows * kKimgDC; e += 256) {
-      const int r = e / kKimgDC, dd = e % kKimgDC, d = d0 + dd;
-      const int i = a * kVRows + r;
-      xs[dd][r] = (i < rows && d < D) ? xc[(size_t)i * D + d] : 0.f;
-    }
-    for (int e = tid; e < kVK * kKimgDC; e += 256) {
-      const int kk = e / kKimgDC, dd = e % kKimgDC, d = d0 + dd, k = c * kVK + kk;
-      ms[dd][kk] = (k < M && d < D) ? mc[(size_t)k * D + d] : 0.f;
-    }
-    __syncthreads();
+      for (int u = 0; u < 8; ++u) acc[q][u] = 0.f;
+    for (int d0 = 0; d0 < D; d0 += kKimgDC) {
+      const int nd = min(kKimgDC, D - d0);
+      __syncthreads();  // the last pass has read its tiles
+      if (D > kKimgDC || c == c0)
+        for (int e = tid; e < kVRows * nd; e += 256) {
+          const int r = e / nd, dd = e - r * nd, i = a * kVRows + r;
+          xs[dd][r] = i < rows ? xc[(size_t)i * D + d0 + dd] : 0.f;
+        }
+      for (int e = tid; e < kVK * nd; e += 256) {
+        const int kk = e / nd, dd = e - kk * nd, k = c * kVK + kk;
+        ms[dd][kk] = k < M ? mc[(size_t)k * D + d0 + dd] : 0.f;
+      }
+      __syncthreads();
 #pragma unroll 4
-    for (int dd = 0; dd < kKimgDC; ++dd) {
-      const float2 x = *reinterpret_cast<const float2 *>(&xs[dd][r0]);
-      const float4 m0 = *reinterpret_cast<const float4 *>(&ms[dd][k0]);
-      const float4 m1 = *reinterpret_cast<const float4 *>(&ms[dd][k0 + 4]);
-      const float mv[8] = {m0.x, m0.y, m0.z, m0.w, m1.x, m1.y, m1.z, m1.w};
+      for (int dd = 0; dd < nd; ++dd) {
+        const float2 x = *reinterpret_cast<const float2 *>(&xs[dd][r0]);
+        const float4 m0 = *reinterpret_cast<const float4 *>(&ms[dd][k0]);
+        const float4 m1 = *reinterpret_cast<const float4 *>(&ms[dd][k0 + 4]);
+        const float mv[8] = {m0.x, m0.y, m0.z, m0.w, m1.x, m1.y, m1.z, m1.w};
 #pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        const float t0 = x.x - mv[u], t1 = x.y - mv[u];
-        acc[0][u] = fmaf(t0, t0, acc[0][u]);
-        acc[1][u] = fmaf(t1, t1, acc[1][u]);
+        for (int u = 0; u < 8; ++u) {
+          const float t0 = x.x - mv[u], t1 = x.y - mv[u];
+          acc[0][u] = fmaf(t0, t0, acc[0][u]);
+          acc[1][u] = fmaf(t1, t1, acc[1][u]);
+        }
       }
     }
-    __syncthreads();
-  }
-  unsigned char *blk = img + ((size_t)a * nch + c) * kVKBlk;
+    unsigned char *blk = img + ((size_t)a * nch + c) * kVKBlk;
 #pragma unroll
-  for (int q = 0; q < 2; ++q) {
-    const int r = r0 + q, i = a * kVRows + r;
-    uint32_t hp[4], lp[4];
+    for (int q = 0; q < 2; ++q) {
+      const int r = r0 + q, i = a * kVRows + r;
+      uint32_t hp[4], lp[4];
 #pragma unroll
-    for (int h = 0; h < 4; ++h) {
-      float w[2];
+      for (int h = 0; h < 4; ++h) {
+        float w[2];
 #pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        const int k = c * kVK + k0 + 2 * h + u;
-        w[u] = (i < rows && k < M) ? (float)kDelta * expf(-0.5f * acc[q][2 * h + u]) : 0.f;
+        for (int u = 0; u < 2; ++u) {
+          const int k = c * kVK + k0 + 2 * h + u;
+          w[u] = (i < rows && k < M) ? (float)kDelta * expf(-0.5f * acc[q][2 * h + u]) : 0.f;
+        }
+        const __nv_bfloat162 hi = __floats2bfloat162_rn(w[0], w[1]);
+        const float2 hf = __bfloat1622float2(hi);
+        hp[h] = *reinterpret_cast<const uint32_t *>(&hi);
+        lp[h] = pack_bf16(w[0] - hf.x, w[1] - hf.y);
       }
-      const __nv_bfloat162 hi = __floats2bfloat162_rn(w[0], w[1]);
-      const float2 hf = __bfloat1622float2(hi);
-      hp[h] = *reinterpret_cast<const uint32_t *>(&hi);
-      lp[h] = pack_bf16(w[0] - hf.x, w[1] - hf.y);
+      const int off = kmajor_off(r, k0, kVK / 8);
+      *reinterpret_cast<uint4 *>(blk + off) = make_uint4(hp[0], hp[1], hp[2], hp[3]);
+      *reinterpret_cast<uint4 *>(blk + kVKHalf + off) = make_uint4(lp[0], lp[1], lp[2], lp[3]);
     }
-    const int off = kmajor_off(r, k0, kVK / 8);
-    *reinterpret_cast<uint4 *>(blk + off) = make_uint4(hp[0], hp[1], hp[2], hp[3]);
-    *reinterpret_cast<uint4 *>(blk + kVKHalf + off) = make_uint4(lp[0], lp[1], lp[2], lp[3]);
   }
 }
 
@@ -577,8 +586,10 @@ gapgb_status variance_enqueue(gapgb_model *m, int S, int N, const int *d_atom_of
       else
         k_var_center<float><<<nb, 256, 0, st>>>(r0, rows, D, (const float *)G, m->d_invth,
                                                 v.d_mu64, (float *)v.xc);
-      k_var_kimg<<<dim3(nch, nA), 256, 0, st>>>(rows, M, D, nch, (const float *)v.xc, v.d_mc32,
-                                                (unsigned char *)v.kbuf);
+      // eight chunks per block, fewer where that left the chip short of blocks
+      const int per = std::max(1, (int)std::min<size_t>(8, (size_t)nch * nA / (8 * device_sms())));
+      k_var_kimg<<<dim3((nch + per - 1) / per, nA), 256, 0, st>>>(
+          rows, M, D, nch, per, (const float *)v.xc, v.d_mc32, (unsigned char *)v.kbuf);
       k_var_tc<<<dim3(nT, nA), kVThreads, kVSmem, st>>>(nch, rows, (const unsigned char *)v.kbuf,
                                                           v.d_qimg, (double *)v.part,
                                                           m->ws.d_flags);
