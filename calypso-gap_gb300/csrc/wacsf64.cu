@@ -657,8 +657,8 @@ __device__ __forceinline__ void finish(const View &s, int i, int cap, int P, con
 // Slot gradients.  split = 1: grid-stride over atoms; a group's scalars pass
 // through the block's own scratch (sc + blockIdx.x * nsc) and are gathered
 // before the next group.  split > 1: block (i, y) writes its units' scalars
-// to sc + i * nsc + (group's first unit) * kUnit and the radial sums to
-// rad[i][slot], for k_w64_gather.
+// to sc + i * nsc + (group's first unit) * kUnit, the radial sums to
+// rad[i][slot] and the groups' first units to first[i][g], for k_w64_gather.
 template <int NAL, int DEG>
 __global__ void __launch_bounds__(kBlk, 4)
     k_w64_bwd(int N, int cap, int capS, const int *__restrict__ cnt,
@@ -667,7 +667,7 @@ __global__ void __launch_bounds__(kBlk, 4)
               const W64Tab *__restrict__ tab, const __grid_constant__ W64Fc fc,
               const u64 *__restrict__ expt, const double *__restrict__ dedg,
               double4 *__restrict__ gslot, double *__restrict__ wvir, double4 *scr,
-              double *__restrict__ rad, size_t nsc, int split) {
+              double *__restrict__ rad, int *__restrict__ first, size_t nsc, int split) {
   constexpr int NB = DEG + 1;
   extern __shared__ __align__(32) unsigned char smraw[];
   const W64Tab &t = *tab;
@@ -731,6 +731,7 @@ __global__ void __launch_bounds__(kBlk, 4)
       __syncthreads();
       double4 *sc = split > 1 ? scr + (size_t)i * nsc + (size_t)u0 * kUnit
                               : scr + (size_t)blockIdx.x * nsc;
+      if (split > 1 && y == 0 && tid == 0) first[i * t.ngrp + g] = u0;
       const int nu = (np + kUnit - 1) / kUnit;
       for (int u = 0; u < nu; ++u) {
         if ((u0 + u) % kClasses % split != y) continue;
@@ -790,7 +791,12 @@ __global__ void __launch_bounds__(kBlk, 4)
   }
 }
 
-// split > 1: the gathers of every group in order, as k_w64_bwd does with split 1
+// split > 1: the gathers that k_w64_bwd does with split 1, a block per atom and
+// group.  Latency bound (a load of 32 bytes and an index search per pair, two
+// threads per slot), so groups in turn cost their sum: 64 carbon atoms with
+// seven groups 133 us by one block per atom.  One group: the block finishes
+// the atom; several: the groups' sums pass through gp[i][g][slot] to
+// k_w64_finish, which adds them in order.
 constexpr int kGatherThreads = 512;
 __global__ void __launch_bounds__(kGatherThreads)
     k_w64_gather(int N, int cap, int capS, const int *__restrict__ cnt,
@@ -798,7 +804,38 @@ __global__ void __launch_bounds__(kGatherThreads)
                  const double4 *__restrict__ apos, const float4 *__restrict__ d32,
                  const W64Tab *__restrict__ tab, const __grid_constant__ W64Fc fc,
                  double4 *__restrict__ gslot, double *__restrict__ wvir, const double4 *scr,
-                 const double *__restrict__ rad, size_t nsc) {
+                 const double *__restrict__ rad, const int *__restrict__ first,
+                 double4 *__restrict__ gp, size_t nsc) {
+  extern __shared__ __align__(32) unsigned char smraw[];
+  const W64Tab &t = *tab;
+  const Lay l = layout(capS, t.nrc, 0);
+  const View s = view(smraw, l);
+  double4 *acc = reinterpret_cast<double4 *>(smraw + l.rest);
+  double *vir = reinterpret_cast<double *>(acc + capS);
+  const int i = blockIdx.x, g = blockIdx.y;
+  const int P = stage<false>(s, t, fc, i, cap, capS, cnt, xyzr, nj, apos, d32, false);
+  for (int q = threadIdx.x; q < P; q += blockDim.x)
+    acc[q] = make_double4(0.0, 0.0, 0.0, gp ? 0.0 : rad[(size_t)i * capS + q]);
+  __syncthreads();
+  if (g < t.ngrp) {  // (a set may have no angular SF)
+    int n;
+    build_pairs<true>(s, t, g, P, n);
+    gather(s, n, scr + (size_t)i * nsc + (size_t)first[i * t.ngrp + g] * kUnit, acc);
+  }
+  __syncthreads();
+  if (gp)
+    for (int q = threadIdx.x; q < P; q += blockDim.x)
+      gp[((size_t)i * t.ngrp + g) * capS + q] = acc[q];
+  else
+    finish(s, i, cap, P, acc, vir, gslot, wvir);
+}
+__global__ void __launch_bounds__(kBlk)
+    k_w64_finish(int cap, int capS, const int *__restrict__ cnt, const double4 *__restrict__ xyzr,
+                 const int *__restrict__ nj, const double4 *__restrict__ apos,
+                 const float4 *__restrict__ d32, const W64Tab *__restrict__ tab,
+                 const __grid_constant__ W64Fc fc, double4 *__restrict__ gslot,
+                 double *__restrict__ wvir, const double *__restrict__ rad,
+                 const double4 *__restrict__ gp) {
   extern __shared__ __align__(32) unsigned char smraw[];
   const W64Tab &t = *tab;
   const Lay l = layout(capS, t.nrc, 0);
@@ -807,15 +844,13 @@ __global__ void __launch_bounds__(kGatherThreads)
   double *vir = reinterpret_cast<double *>(acc + capS);
   const int i = blockIdx.x;
   const int P = stage<false>(s, t, fc, i, cap, capS, cnt, xyzr, nj, apos, d32, false);
-  for (int q = threadIdx.x; q < P; q += blockDim.x)
-    acc[q] = make_double4(0.0, 0.0, 0.0, rad[(size_t)i * capS + q]);
-  int u0 = 0;
-  for (int g = 0; g < t.ngrp; ++g) {
-    __syncthreads();
-    int n;
-    const int np = build_pairs<true>(s, t, g, P, n);
-    gather(s, n, scr + (size_t)i * nsc + (size_t)u0 * kUnit, acc);
-    u0 += (np + kUnit - 1) / kUnit;
+  for (int q = threadIdx.x; q < P; q += kBlk) {
+    double4 a = make_double4(0.0, 0.0, 0.0, rad[(size_t)i * capS + q]);
+    for (int g = 0; g < t.ngrp; ++g) {
+      const double4 v = gp[((size_t)i * t.ngrp + g) * capS + q];
+      a = make_double4(a.x + v.x, a.y + v.y, a.z + v.z, a.w + v.w);
+    }
+    acc[q] = a;
   }
   __syncthreads();
   finish(s, i, cap, P, acc, vir, gslot, wvir);
@@ -1245,7 +1280,8 @@ void launch_w64_bwd(const gapgb_model *m, Workspace &ws, int N, int cap, int cap
   int split = split_of(N);
   size_t nsc = group_units(capS) * kUnit * std::max(1, t.ngrp), need = 0;
   if (split > 1) {
-    need = (size_t)N * (nsc * 32 + (size_t)capS * 8);
+    need = (size_t)N * (nsc * 32 + (t.ngrp > 1 ? (size_t)t.ngrp * capS * 32 : 0) +
+                        (size_t)capS * 8 + (size_t)t.ngrp * 4);
     if (need > kScratchMax || !scratch(m, ws, need, st)) split = 1;
   }
   int gx = N;
@@ -1256,17 +1292,30 @@ void launch_w64_bwd(const gapgb_model *m, Workspace &ws, int N, int cap, int cap
     if (!scratch(m, ws, gx * nsc * 32, st)) gx = (int)(ws.w64_bytes / (nsc * 32));  // >= 1: w64_applies
   }
   double4 *sc = (double4 *)ws.w64_scratch;
-  double *rad = (double *)(sc + (split > 1 ? (size_t)N * nsc : 0));
+  // split > 1: scalars [N][nsc], group sums [N][ngrp][capS], radial sums, first units
+  double4 *gp = split > 1 ? sc + (size_t)N * nsc : nullptr;
+  double *rad = (double *)(gp + (split > 1 && t.ngrp > 1 ? (size_t)N * t.ngrp * capS : 0));
+  int *first = (int *)(rad + (split > 1 ? (size_t)N * capS : 0));
+  if (t.ngrp <= 1) gp = nullptr;
   b<<<dim3(gx, split), kBlk, smem, st>>>(N, cap, capS, ws.nbr_cnt, ws.nbr_xyz, ws.nbr_j, ws.apos,
                                          ws.nbr_d32, m->d_w64, m->w64h.fc, m->d_exp64,
                                          (const double *)ws.dedg, (double4 *)ws.gslot, ws.wvir, sc,
-                                         rad, nsc, split);
+                                         rad, first, nsc, split);
   if (split > 1) {
     const size_t sg = layout(capS, t.nrc, (size_t)capS * 32 + 36 * 8).total;
     kernel_smem((const void *)k_w64_gather, (int)sg, true);
-    k_w64_gather<<<N, kGatherThreads, sg, st>>>(N, cap, capS, ws.nbr_cnt, ws.nbr_xyz, ws.nbr_j,
-                                                ws.apos, ws.nbr_d32, m->d_w64, m->w64h.fc,
-                                                (double4 *)ws.gslot, ws.wvir, sc, rad, nsc);
+    // two threads per slot: few slots, small blocks (512 alloy atoms, 56 slots:
+    // 43 us at 512 threads)
+    const int th = std::min(kGatherThreads, std::max(kBlk, (2 * capS + 63) / 64 * 64));
+    k_w64_gather<<<dim3(N, std::max(1, t.ngrp)), th, sg, st>>>(
+        N, cap, capS, ws.nbr_cnt, ws.nbr_xyz, ws.nbr_j, ws.apos, ws.nbr_d32, m->d_w64, m->w64h.fc,
+        (double4 *)ws.gslot, ws.wvir, sc, rad, first, gp, nsc);
+    if (gp) {
+      kernel_smem((const void *)k_w64_finish, (int)sg, true);
+      k_w64_finish<<<N, kBlk, sg, st>>>(cap, capS, ws.nbr_cnt, ws.nbr_xyz, ws.nbr_j, ws.apos,
+                                        ws.nbr_d32, m->d_w64, m->w64h.fc, (double4 *)ws.gslot,
+                                        ws.wvir, rad, gp);
+    }
   }
 }
 
