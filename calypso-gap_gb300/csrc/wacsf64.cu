@@ -30,8 +30,8 @@
 // descriptors and 55 for the gradient, where the generic kernels issue about
 // 520 and 770.  Measured (ncu, both generic kernels -> these, split launches
 // included): 512 alloy atoms (56 slots, 690 pairs each) 520 -> 82 us and
-// 665 -> 145 us; 64 carbon atoms (158 slots, 7 cutoffs) 2380 -> 102 us and
-// 1858 -> 259 us; 6.4 k atoms of ragged cells 5444 -> 604 and 10177 -> 1094
+// 665 -> 133 us; 64 carbon atoms (158 slots, 7 cutoffs) 2380 -> 102 us and
+// 1858 -> 211 us; 6.4 k atoms of ragged cells 5444 -> 604 and 10177 -> 1094
 // us (842 and 1330 with the geometry and the exponential's argument in FP64,
 // 1139 and 1691 with all of the polynomials there).
 //
@@ -794,7 +794,7 @@ __global__ void __launch_bounds__(kBlk, 4)
 // split > 1: the gathers that k_w64_bwd does with split 1, a block per atom and
 // group.  Latency bound (a load of 32 bytes and an index search per pair, two
 // threads per slot), so groups in turn cost their sum: 64 carbon atoms with
-// seven groups 133 us by one block per atom.  One group: the block finishes
+// seven groups 133 us by one block per atom, 70 + 14 us so.  One group: the block finishes
 // the atom; several: the groups' sums pass through gp[i][g][slot] to
 // k_w64_finish, which adds them in order.
 constexpr int kGatherThreads = 512;
@@ -1305,7 +1305,7 @@ void launch_w64_bwd(const gapgb_model *m, Workspace &ws, int N, int cap, int cap
     const size_t sg = layout(capS, t.nrc, (size_t)capS * 32 + 36 * 8).total;
     kernel_smem((const void *)k_w64_gather, (int)sg, true);
     // two threads per slot: few slots, small blocks (512 alloy atoms, 56 slots:
-    // 43 us at 512 threads)
+    // 31 us at 128 threads, 43 at 512)
     const int th = std::min(kGatherThreads, std::max(kBlk, (2 * capS + 63) / 64 * 64));
     k_w64_gather<<<dim3(N, std::max(1, t.ngrp)), th, sg, st>>>(
         N, cap, capS, ws.nbr_cnt, ws.nbr_xyz, ws.nbr_j, ws.apos, ws.nbr_d32, m->d_w64, m->w64h.fc,
