@@ -47,8 +47,8 @@ def parse():
     p.add_argument("--warmup", type=int, default=3)
     p.add_argument("--impl", default="gapgb", choices=["gapgb", "reference"])
     p.add_argument("--batch", type=int, default=None,
-                   help="structures per step per GPU (default: one full wave of the tensor-core "
-                        "GPR, two 128-atom CTAs per SM: 76 alloy512 cells on 152 SMs)")
+                   help="structures per step per GPU (default: a full wave of the tensor-core GPR "
+                        "in each of two pipelines, 128 atoms per SM: 76 alloy512 cells on 152 SMs)")
     p.add_argument("--precision", default="tc", choices=["fp32", "tc", "tf32", "fp64", "mixed"])
     p.add_argument("--no-oracle", action="store_true", help="skip the oracle error check")
     p.add_argument("--pipelines", type=int, default=2, choices=[1, 2],
@@ -100,9 +100,9 @@ def shard_seeds(rank, batch):
 
 
 def default_batch(args, device):
-    """Structures per step: by default one full wave of the tensor-core GPR
-    kernel, which holds 128 atoms per CTA and two CTAs per SM (76 alloy512
-    cells = 38912 atoms on 152 SMs)."""
+    """Structures per step: by default a full wave of the tensor-core GPR kernel
+    (128 atoms per CTA, one CTA per SM) in each of the two pipelines (76
+    alloy512 cells = 38912 atoms on 152 SMs)."""
     if args.batch is None:
         import torch
         sms = torch.cuda.get_device_properties(device).multi_processor_count
@@ -1359,10 +1359,11 @@ def run_fit(args):
             "heldout_rmse_eV_per_atom": float(np.sqrt(np.mean(((Eh - Eh_t) / 512) ** 2))),
             "teacher_energy_scale_eV_per_atom": float(np.abs(Eh_t / 512).max()),
             "coeff_max": float(np.abs(c).max()),
-            # per call: prep x2, neighbour build, reverse, FP64 descriptors, K_MM, jitter,
-            # weights, design rows, Gram, right-hand side, 3 per Cholesky panel (2 for the
-            # last), solves
-            "gpu_launches": (5 + 6 + 3 * ((len(mm) + 63) // 64) - 2 + 1) * len(times)}
+            # per call, at least: prep x2, neighbour build x2, FP64 descriptors; K_MM and the
+            # design rows 3 each (more chunks for large sets), jitter, weights, Gram,
+            # right-hand side; per Cholesky block the diagonal, panel, two updates (none
+            # below the last block, one below the last but one) and back substitution
+            "gpu_launches": (5 + 6 + 4 + 5 * ((len(mm) + 63) // 64) - 4) * len(times)}
     print(json.dumps(line), flush=True)
 
 
@@ -1560,7 +1561,8 @@ def main():
         "data": "synthetic",
         "config": {"workload": "alloy512 ternary fcc (Z 13/28/40), D=64, M=4000",
                    "structures_per_step": S, "atoms_per_step_per_gpu": N,
-                   "batch_rule": "one wave of the tensor-core GPR: 2 CTAs x 128 atoms per SM",
+                   "batch_rule": "a wave of the tensor-core GPR in each of two pipelines: 2 x 128 "
+                                 "atoms per SM",
                    "precision": args.precision, "pipelines": args.pipelines,
                    "l2": "flushed between steps (512 MB write)"},
         "e2e": {"value": world * N / e2e_s, "unit": UNIT, "h2d_bytes_per_step": int(h2d),
