@@ -476,7 +476,7 @@ __global__ void __launch_bounds__(kThreads, 1)
           const bool in = zf > -1020.f;
           const int n = (int)(z >> 52);
           const u64 m = exp2_fix((u64)z & ((1ull << 52) - 1), T);
-          u64 bits = ((u64)(uint32_t)(n + 1022) << 52) + ((m + 1024) >> 11);
+          u64 bits = ((u64)(uint32_t)(n + 1022) << 52) + (m >> 11) + ((m >> 10) & 1);
           bits |= (u64)(c.es & 0x80000000u) << 32;
           if (in) emax = max(emax, n);
           out[(size_t)(8 * g + q) * kR] = in ? __longlong_as_double((i64)bits) : 0.0;

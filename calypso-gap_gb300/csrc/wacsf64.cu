@@ -144,9 +144,11 @@ __device__ __forceinline__ double exp_neg(const W64Exp &c, u64 x, int e,
   const uint32_t y4 = __umulhi(y3, yh);                    // 2^-72
   const u64 p = y + (y2 >> 11) +
                 ((u64)(__umulhi(y3, 0x2AAAAAABu) + (__umulhi(y4, 0x0AAAAAABu) >> 10)) << 12);
+  // rounded after the shift: at a zero argument m is 55 below 2^64, m + 1024
+  // would wrap, and the carry into the exponent is what makes the result 1
   const u64 m = t + (__umul64hi(t, p) >> 10);
   return __longlong_as_double(
-      (i64)(((u64)(uint32_t)((k >> 10) + 1022) << 52) + ((m + 1024) >> 11)));
+      (i64)(((u64)(uint32_t)((k >> 10) + 1022) << 52) + (m >> 11) + ((m >> 10) & 1)));
 }
 
 // sums v[0..N) over the warp's lanes by halving exchanges: at each step a
