@@ -28,24 +28,24 @@ static thread_local std::string g_last_error;
 
 void set_last_error(const std::string &s) { g_last_error = s; }
 
-bool grow_scratch(const gapgb_model *m, void **p, size_t *have, size_t bytes, cudaStream_t st) {
-  if (bytes <= *have) return true;
+bool grow_scratch(Workspace &ws, void **p, size_t *have, size_t want, size_t need,
+                  cudaStream_t st) {
+  if (want <= *have) return true;
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  if (m->live_graphs->load() > 0 || cudaStreamIsCapturing(st, &cap) != cudaSuccess ||
-      cap != cudaStreamCaptureStatusNone)
-    return false;
-  const size_t had = *have;
-  if (*p) cudaFree(*p);
-  for (const size_t b : {bytes, had}) {  // the old size again when the new one fails
-    *p = nullptr;
-    *have = 0;
-    if (b > 0 && cudaMalloc(p, b) == cudaSuccess) {
+  if (cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone)
+    return need <= *have;
+  // half as much again, so that the retired buffers stay below twice the last
+  for (const size_t b : {std::max(want, *have + *have / 2), need}) {
+    void *q = nullptr;
+    if (b > *have && cudaMalloc(&q, b) == cudaSuccess) {
+      if (*p) ws.retired.push_back(*p);
+      *p = q;
       *have = b;
       break;
     }
     cudaGetLastError();
   }
-  return *have >= bytes;
+  return need <= *have;
 }
 
 namespace {
@@ -104,6 +104,8 @@ void free_ws(Workspace &ws) {
   ws.w64_bytes = 0;
   free_dev(ws.g64_scratch);
   ws.g64_bytes = 0;
+  for (void *p : ws.retired) cudaFree(p);
+  ws.retired.clear();
   ws.tc_scratch_size = 0;
   if (ws.h_flags) cudaFreeHost(ws.h_flags);
   ws.h_flags = nullptr;

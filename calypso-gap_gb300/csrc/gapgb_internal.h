@@ -334,6 +334,7 @@ struct Workspace {
   size_t w64_bytes = 0;
   void *g64_scratch = nullptr;  // gpr64_tc.cu: operands, kernel values, partial sums
   size_t g64_bytes = 0;
+  std::vector<void *> retired;  // outgrown scratch that captured graphs may hold (grow_scratch)
   // contributing angular pairs (j | k << 8) of every atom, recorded by the
   // grouped FP32 descriptor kernel and streamed by its gradient kernel
   unsigned short *pairs = nullptr;  // [N][kPairCap]
@@ -473,10 +474,14 @@ void launch_refresh(Workspace &ws, int N, int cap, cudaStream_t st, bool exact =
 template <typename T>
 void launch_wacsf_fwd(const gapgb_model *m, Workspace &ws, int N, int cap, int cap_smem,
                       cudaStream_t st, int a0 = 0, int a1 = -1);
-// A kernel's scratch in the workspace, grown as needed.  False when it cannot
-// be had: an allocation failed, the buffer would move while a captured graph
-// holds its address, or the stream is being captured (no allocation there).
-bool grow_scratch(const gapgb_model *m, void **p, size_t *have, size_t bytes, cudaStream_t st);
+// A kernel's scratch in the workspace: `want` bytes (what any batch up to the
+// workspace's size may take, so that no smaller batch grows it), at least
+// `need`.  False when `need` cannot be had: the allocation failed, or the stream is being
+// captured and no call before has sized the buffer.  A captured graph may hold
+// the address of a buffer that is outgrown: it is kept until the workspace
+// itself is reallocated.
+bool grow_scratch(Workspace &ws, void **p, size_t *have, size_t want, size_t need,
+                  cudaStream_t st);
 // gpr64_tc.cu: the FP64 GPR on the tensor cores
 gapgb_status g64_prepare(gapgb_model *m, bool refresh = false);
 template <typename TG>

@@ -851,7 +851,7 @@ gapgb_status g64_prepare(gapgb_model *m, bool refresh) {
 // scratch of one launch over N atoms: operands of all of them, kernel values
 // and partial sums of `ct` row tiles at a time
 struct G64Run {
-  int tiles, ct, sa, sb;
+  int tiles, ct, sa, sb, slots;
   size_t xh, img, row, rowexp, W, part, epart, bytes;
 };
 static G64Run g64_run(const G64 &g, int N, int D) {
@@ -863,6 +863,9 @@ static G64Run g64_run(const G64 &g, int N, int D) {
   r.ct = (int)std::max<size_t>(1, std::min<size_t>({(size_t)r.tiles, (size_t)sms, ((size_t)768 << 20) / per}));
   r.sa = std::max(1, std::min(g.nt1, sms / r.ct));
   r.sb = std::max(1, std::min(g.nst / kDrain, sms / (r.ct * g.nz)));
+  // partial sums: the most that any batch up to N takes (sb ct is not monotone
+  // in N), so that a smaller batch fits into a larger one's scratch
+  r.slots = std::max(r.ct, std::min(r.ct * (g.nst / kDrain), sms / g.nz));
   size_t o = 0;
   auto take = [&](size_t &at, size_t n) { at = o, o += up256(n); };
   take(r.xh, 8 * (size_t)N * D);
@@ -870,10 +873,15 @@ static G64Run g64_run(const G64 &g, int N, int D) {
   take(r.row, sizeof(Row) * (size_t)r.tiles * kR);
   take(r.rowexp, 4 * (size_t)r.tiles * kR);
   take(r.W, per * r.ct);
-  take(r.part, sizeof(longlong2) * (size_t)g.nz * r.sb * r.ct * kN2 * kR);
-  take(r.epart, sizeof(longlong2) * (size_t)r.sb * r.ct * 2 * kR);
+  take(r.part, sizeof(longlong2) * (size_t)g.nz * r.slots * kN2 * kR);
+  take(r.epart, sizeof(longlong2) * (size_t)r.slots * 2 * kR);
   r.bytes = o;
   return r;
+}
+
+static bool g64_scratch(const G64 &g, Workspace &ws, int N, int D, const G64Run &r, cudaStream_t st) {
+  return grow_scratch(ws, &ws.g64_scratch, &ws.g64_bytes, g64_run(g, std::max(N, ws.N), D).bytes,
+                      r.bytes, st);
 }
 
 // The FP64 GPR of N atoms; false (nothing launched) when the model has no
@@ -884,7 +892,7 @@ bool launch_gpr64(const gapgb_model *m, Workspace &ws, int N, cudaStream_t st) {
   const int M = m->host.M, D = m->host.D;
   const G64 g = g64_layout(M, D);
   const G64Run r = g64_run(g, N, D);
-  if (!grow_scratch(m, &ws.g64_scratch, &ws.g64_bytes, r.bytes, st)) return false;
+  if (!g64_scratch(g, ws, N, D, r, st)) return false;
   const unsigned char *p = m->d_g64;
   unsigned char *q = (unsigned char *)ws.g64_scratch;
   Row *row = (Row *)(q + r.row);
@@ -921,7 +929,7 @@ static bool g64_kernel_values(const gapgb_model *m, Workspace &ws, int N, const 
   const int M = m->host.M, D = m->host.D;
   const G64 g = g64_layout(M, D);
   const G64Run r = g64_run(g, N, D);
-  if (!grow_scratch(m, &ws.g64_scratch, &ws.g64_bytes, r.bytes, st)) return false;
+  if (!g64_scratch(g, ws, N, D, r, st)) return false;
   const unsigned char *p = m->d_g64;
   unsigned char *q = (unsigned char *)ws.g64_scratch;
   Row *row = (Row *)(q + r.row);

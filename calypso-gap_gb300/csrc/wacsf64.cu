@@ -1237,19 +1237,55 @@ size_t group_units(int capS) {
 }
 
 constexpr size_t kScratchMax = (size_t)1 << 30;
-bool scratch(const gapgb_model *m, Workspace &ws, size_t bytes, cudaStream_t st) {
-  return grow_scratch(m, &ws.w64_scratch, &ws.w64_bytes, bytes, st);
+
+// Scratch of one launch.  Descriptors: the moments of N atoms, split.
+size_t fwd_bytes(const W64Tab &t, int N) {
+  return sizeof(double) * (size_t)N * t.ngrp * kClasses * 2 * t.nal * (t.deg + 1);
+}
+// Gradient, split: scalars [N][nsc], group sums [N][ngrp][capS], radial sums,
+// first units.
+size_t split_nsc(const W64Tab &t, int capS) {
+  return group_units(capS) * kUnit * std::max(1, t.ngrp);
+}
+size_t bwd_bytes(const W64Tab &t, int N, int capS) {
+  return (size_t)N * (split_nsc(t, capS) * 32 + (t.ngrp > 1 ? (size_t)t.ngrp * capS * 32 : 0) +
+                      (size_t)capS * 8 + (size_t)t.ngrp * 4);
+}
+// Gradient, one block per atom: a region per resident block.
+size_t region_bytes(int capS) { return group_units(capS) * kUnit * 32; }
+int resident(const W64Tab &t, int N, int capS, size_t smem) {
+  Fwd f;
+  Bwd b;
+  pick(t.nal, t.deg, &f, &b);
+  kernel_smem((const void *)b, (int)smem, true);
+  const int gx = std::min(N, device_sms() * kernel_occupancy((const void *)b, kBlk, smem));
+  return (int)std::min<size_t>(gx, std::max<size_t>(1, kScratchMax / region_bytes(capS)));
+}
+// The most that any batch of up to N atoms with capS slots takes.  A launch
+// splits atoms only below kScratchMax; the largest batch of each split bounds
+// the smaller ones.
+size_t scratch_bound(const gapgb_model *m, int N, int capS) {
+  const W64Tab &t = m->w64h;
+  size_t b = resident(t, N, capS, bwd_smem(m, capS)) * region_bytes(capS);
+  for (int s = 2; s <= kClasses; s *= 2) {
+    const int n = std::min(N, (8 * device_sms() - 1) / (s / 2));  // the most atoms that take s
+    b = std::max(b, std::min(kScratchMax, std::max(fwd_bytes(t, n), bwd_bytes(t, n, capS))));
+  }
+  return b;
 }
 
 }  // namespace
 
-// Whether the kernels take a batch with capS slots per atom.  Also sizes the
-// scratch of the gradient's launch with one block per atom (a region per
-// resident block, fewer blocks when a region is large), so that the gradient
-// of a batch always takes the kernels that its descriptors took.
+// Whether the kernels take a batch with capS slots per atom.  Also sizes their
+// scratch: at least a region of the gradient's launch with one block per atom, so
+// that the gradient of a batch always takes the kernels that its descriptors
+// took; the launches split atoms, or keep more blocks resident, as far as it
+// reaches (the results are the same).
 bool w64_applies(const gapgb_model *m, Workspace &ws, int capS, cudaStream_t st) {
   return m->d_w64 && capS < 65536 && fwd_smem(m, capS) <= kSmemMax &&
-         bwd_smem(m, capS) <= kSmemMax && scratch(m, ws, group_units(capS) * kUnit * 32, st);
+         bwd_smem(m, capS) <= kSmemMax &&
+         grow_scratch(ws, &ws.w64_scratch, &ws.w64_bytes, scratch_bound(m, ws.N, capS),
+                      region_bytes(capS), st);
 }
 
 void launch_w64_fwd(const gapgb_model *m, Workspace &ws, int N, int cap, int capS, cudaStream_t st) {
@@ -1260,9 +1296,8 @@ void launch_w64_fwd(const gapgb_model *m, Workspace &ws, int N, int cap, int cap
   pick(t.nal, t.deg, &f, &b);
   const size_t smem = fwd_smem(m, capS);
   kernel_smem((const void *)f, (int)smem, true);
-  const size_t need = sizeof(double) * (size_t)N * t.ngrp * kClasses * NM;
   int split = split_of(N);
-  if (split > 1 && (need > kScratchMax || !scratch(m, ws, need, st))) split = 1;
+  if (fwd_bytes(t, N) > std::min(kScratchMax, ws.w64_bytes)) split = 1;
   const int gx = std::min(N, 1 << 20);
   f<<<dim3(gx, split), kBlk, smem, st>>>(N, cap, capS, ws.nbr_cnt, ws.nbr_xyz, ws.nbr_j, ws.apos,
                                          ws.nbr_d32, m->d_w64, m->w64h.fc, m->d_exp64,
@@ -1279,22 +1314,14 @@ void launch_w64_bwd(const gapgb_model *m, Workspace &ws, int N, int cap, int cap
   pick(t.nal, t.deg, &f, &b);
   const size_t smem = bwd_smem(m, capS);
   kernel_smem((const void *)b, (int)smem, true);
-  int split = split_of(N);
-  size_t nsc = group_units(capS) * kUnit * std::max(1, t.ngrp), need = 0;
-  if (split > 1) {
-    need = (size_t)N * (nsc * 32 + (t.ngrp > 1 ? (size_t)t.ngrp * capS * 32 : 0) +
-                        (size_t)capS * 8 + (size_t)t.ngrp * 4);
-    if (need > kScratchMax || !scratch(m, ws, need, st)) split = 1;
-  }
-  int gx = N;
+  int split = split_of(N), gx = N;
+  size_t nsc = split_nsc(t, capS);
+  if (bwd_bytes(t, N, capS) > std::min(kScratchMax, ws.w64_bytes)) split = 1;
   if (split == 1) {
     nsc = group_units(capS) * kUnit;
-    gx = std::min(N, device_sms() * kernel_occupancy((const void *)b, kBlk, smem));
-    gx = (int)std::min<size_t>(gx, std::max<size_t>(1, kScratchMax / (nsc * 32)));
-    if (!scratch(m, ws, gx * nsc * 32, st)) gx = (int)(ws.w64_bytes / (nsc * 32));  // >= 1: w64_applies
+    gx = (int)std::min<size_t>(resident(t, N, capS, smem), ws.w64_bytes / region_bytes(capS));
   }
   double4 *sc = (double4 *)ws.w64_scratch;
-  // split > 1: scalars [N][nsc], group sums [N][ngrp][capS], radial sums, first units
   double4 *gp = split > 1 ? sc + (size_t)N * nsc : nullptr;
   double *rad = (double *)(gp + (split > 1 && t.ngrp > 1 ? (size_t)N * t.ngrp * capS : 0));
   int *first = (int *)(rad + (split > 1 ? (size_t)N * capS : 0));
@@ -1334,7 +1361,8 @@ bool launch_w64_jac(const gapgb_model *m, Workspace &ws, int N, int cap, int cap
   kernel_smem((const void *)f, (int)smem, true);
   int gx = std::min(N, device_sms() * kernel_occupancy((const void *)f, kBlk, smem));
   gx = (int)std::min<size_t>(gx, std::max<size_t>(1, kScratchMax / (nsc * 32)));
-  if (!scratch(m, ws, gx * nsc * 32, st)) return false;
+  if (!grow_scratch(ws, &ws.w64_scratch, &ws.w64_bytes, gx * nsc * 32, gx * nsc * 32, st))
+    return false;
   f<<<gx, kBlk, smem, st>>>(N, cap, capS, ws.nbr_cnt, ws.nbr_xyz, ws.nbr_j, ws.apos, ws.nbr_d32,
                             m->d_w64, t.fc, m->d_exp64, J, (double4 *)ws.w64_scratch, nsc, na);
   return true;
