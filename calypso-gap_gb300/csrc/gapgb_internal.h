@@ -383,6 +383,7 @@ struct gapgb_model {
   int tf32_tiles = 0;
   unsigned char *d_g64 = nullptr;      // digit images of the FP64 tensor-core GPR (gpr64_tc.cu)
   bool g64_tried = false;              // g64_prepare ran (d_g64 stays null: the model does not qualify)
+  bool g64_finite = false;             // every coefficient is finite
   int device = 0;
   int precision = GAPGB_PREC_FP64;
   int cap = 256;

@@ -802,6 +802,7 @@ gapgb_status g64_prepare(gapgb_model *m, bool refresh) {
   if (refresh && !m->d_g64) return GAPGB_OK;
   if (!refresh && m->g64_tried) return GAPGB_OK;
   m->g64_tried = true;
+  m->g64_finite = std::all_of(h.coeff.begin(), h.coeff.end(), [](double c) { return std::isfinite(c); });
   const int M = h.M, D = h.D;
   if (D > 80) return GAPGB_OK;
   const G64 g = g64_layout(M, D);
@@ -885,10 +886,11 @@ static bool g64_scratch(const G64 &g, Workspace &ws, int N, int D, const G64Run 
 }
 
 // The FP64 GPR of N atoms; false (nothing launched) when the model has no
-// image or the scratch cannot be had (grow_scratch).
+// image, a coefficient is not finite (fixed point has no NaN: the CUDA-core
+// kernel carries it into the results) or the scratch cannot be had (grow_scratch).
 template <typename TG>
 bool launch_gpr64(const gapgb_model *m, Workspace &ws, int N, cudaStream_t st) {
-  if (!m->d_g64) return false;
+  if (!m->d_g64 || !m->g64_finite) return false;
   const int M = m->host.M, D = m->host.D;
   const G64 g = g64_layout(M, D);
   const G64Run r = g64_run(g, N, D);
