@@ -440,7 +440,9 @@ __global__ void __launch_bounds__(kThreads, 1)
     const u64 *T = reinterpret_cast<const u64 *>(sm + oT);
     int emax = INT_MIN;
     for (int t = 0; t < nt; ++t) {
-      if (!mbar_wait(dfull + 8 * (t & 1), (t >> 1) & 1, flags) || *abort_flag) {
+      // (a warp gives up as one: the TMEM loads and __syncwarp below need all of it)
+      if (!__all_sync(0xffffffffu, mbar_wait(dfull + 8 * (t & 1), (t >> 1) & 1, flags) &&
+                                       !*abort_flag)) {
         *abort_flag = 1;
         break;
       }
@@ -598,8 +600,10 @@ __global__ void __launch_bounds__(kThreads, 1)
 #pragma unroll
         for (int q = 0; q < 16; ++q) nx[q] = w[((size_t)(s + 1) * kT2 + q) * kR];
       }
-      if (s >= 2) ok = mbar_wait(sempty + 8 * (s & 1), ((s >> 1) - 1) & 1, flags);
-      if (!ok || *abort_flag) break;
+      // (a warp gives up as one, here and below)
+      ok = s < 2 || mbar_wait(sempty + 8 * (s & 1), ((s >> 1) - 1) & 1, flags);
+      ok = __all_sync(0xffffffffu, ok && !*abort_flag) != 0;
+      if (!ok) break;
       unsigned char *dst = sm + (s & 1) * kA2;
 #pragma unroll
       for (int g = 0; g < 2; ++g) {
@@ -622,8 +626,8 @@ __global__ void __launch_bounds__(kThreads, 1)
       __syncwarp();
       if (lane == 0) mbar_arrive(afull + 8 * (s & 1));
       if (s % kDrain == kDrain - 1 || s == ns - 1) {
-        ok = mbar_wait(dfull, (s / kDrain) & 1, flags);
-        if (!ok || *abort_flag) break;
+        ok = __all_sync(0xffffffffu, mbar_wait(dfull, (s / kDrain) & 1, flags) && !*abort_flag) != 0;
+        if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
         for (int g = 0; g < 4; ++g) {

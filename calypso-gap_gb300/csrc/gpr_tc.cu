@@ -367,7 +367,7 @@ __global__ void __launch_bounds__(kGprThreads, 1)
     sync16();
     if (set == 0 && half == 0) ep[row] = emine + ep[row];
     sync16();
-    if (!*abort_flag) {
+    if (__all_sync(0xffffffffu, !*abort_flag)) {  // (the TMEM load needs the whole warp)
       // dE/dG: each thread a row and 16 components
       const double etot = ep[row];
       const int d0 = half * 32 + set * 16;
