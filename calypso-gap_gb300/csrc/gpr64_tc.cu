@@ -404,7 +404,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       int loaded = 0, waited = 0;
       for (; loaded < NB && loaded < nt; ++loaded) load(loaded);
       bool ok = true;
-      int t = 0;
+      int t = 0, issued = 0;  // tiles whose MMAs are under way
       for (; t < nt && ok; ++t) {
         ok = mbar_wait(bfull + 8 * (t % NB), (t / NB) & 1, flags);
         if (!ok) break;
@@ -420,6 +420,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                  (kk > 0 || i > 0) ? 1u : 0u);
         umma_commit(dfull + 8 * (t & 1));
         umma_commit(bempty + 8 * (t % NB));
+        issued = t + 1;
         const int f = t - (NB - 1);  // the tile whose buffer is refilled
         if (loaded < nt && f >= 0) {
           ok = mbar_wait(bempty + 8 * (f % NB), (f / NB) & 1, flags);
@@ -428,9 +429,10 @@ __global__ void __launch_bounds__(kThreads, 1)
         }
       }
       if (t < nt) *abort_flag = 1;
-      // a wait gave up: one more bounded wait for each copy still in flight
+      // a wait gave up: one more bounded wait for each copy still in flight; and
+      // for the last MMAs, before the tensor memory goes
       for (; waited < loaded; ++waited) mbar_wait(bfull + 8 * (waited % NB), (waited / NB) & 1, flags);
-      if (t > 0) mbar_wait(bempty + 8 * ((t - 1) % NB), ((t - 1) / NB) & 1, flags);
+      if (issued > 0) mbar_wait(bempty + 8 * ((issued - 1) % NB), ((issued - 1) / NB) & 1, flags);
     }
   } else {
     const int quad = warp & 3, half = warp >> 2;
@@ -544,7 +546,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       int loaded = 0, waited = 0;
       for (; loaded < 2 && loaded < ns; ++loaded) load(loaded);
       bool ok = true;
-      int s = 0;
+      int s = 0, issued = 0;
       for (; s < ns && ok; ++s) {
         ok = mbar_wait(bfull + 8 * (s & 1), (s >> 1) & 1, flags);
         if (!ok) break;
@@ -567,6 +569,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                    instr_desc(kR, n - 256), acc);
           }
         umma_commit(sempty + 8 * (s & 1));
+        issued = s + 1;
         if (s % kDrain == kDrain - 1 || s == ns - 1) umma_commit(dfull);
         if (loaded < ns && s > 0) {
           ok = mbar_wait(sempty + 8 * ((s - 1) & 1), ((s - 1) >> 1) & 1, flags);
@@ -576,7 +579,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       }
       if (s < ns) *abort_flag = 1;
       for (; waited < loaded; ++waited) mbar_wait(bfull + 8 * (waited & 1), (waited >> 1) & 1, flags);
-      if (s > 0) mbar_wait(sempty + 8 * ((s - 1) & 1), ((s - 1) >> 1) & 1, flags);
+      if (issued > 0) mbar_wait(sempty + 8 * ((issued - 1) & 1), ((issued - 1) >> 1) & 1, flags);
     }
   } else {
     const int quad = warp & 3, half = warp >> 2;
