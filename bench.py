@@ -1124,15 +1124,14 @@ def run_md(args):
                 "t_end": {"dE_per_atom": float(abs(Et[0] - Ep[0]) / N),
                           "dF_max": float(np.abs(Ft - Fp).max()),
                           "dstress_max_GPa": float(np.abs(St - Sp).max())}},
-            # per step: kick+drift, wrap or skin check, prep of the atoms (and
-            # of the cell, at a rebuild), refresh,
+            # per step: kick+drift, wrap or skin check, prep x2, refresh,
             # descriptors, tensor-core GPR (prep + kernel), slot gradients with
-            # the force scatter, structure sums x2, kick, kinetic sums x2 = 13,
+            # the force scatter, structure sums x2, kick, kinetic sums x2 = 14,
             # plus 4 for the second pipeline of a large batch; a rebuild step
-            # adds the cell's prep, the build, the bins (offsets, count, scan,
-            # fill) and the binned build in place of the refresh (+6)
-            "gpu_launches": (13 + step_kernels("tc", N) - 9) * args.md_steps
-                            + 6 * (args.md_steps // 10),
+            # adds the build, the bins (offsets, count, scan, fill) and the
+            # binned build in place of the refresh (+5)
+            "gpu_launches": (14 + step_kernels("tc", N) - 9) * args.md_steps
+                            + 5 * (args.md_steps // 10),
             "clocks": tc["clocks"]}
     print(json.dumps(line), flush=True)
 

@@ -637,9 +637,8 @@ gapgb_status md_eval_enqueue(gapgb_model *m, int S, int N, const int *d_atom_off
   Workspace &ws = m->ws;
   const double rb = m->host.rcut + skin;
   GAPGB_CUDA_TRY(cudaMemsetAsync(ws.d_flags + 1, 0, 2 * sizeof(int), s));
-  // between rebuilds the cells and the cutoff are those of the last rebuild
-  launch_prep(m, ws, S, N, d_atom_off, d_species, d_lat, d_pos, rb, s, rebuild && N >= kBinMinAtoms,
-              rebuild);
+  // (the caller may have strained its cells since the last rebuild)
+  launch_prep(m, ws, S, N, d_atom_off, d_species, d_lat, d_pos, rb, s, rebuild && N >= kBinMinAtoms);
   if (rebuild) launch_neighbors(ws, S, N, N, m->cap, rb, s, m->precision == GAPGB_PREC_FP64);
   else launch_refresh(ws, N, m->cap, s, m->precision == GAPGB_PREC_FP64);
   return enqueue_tail(m, S, N, m->cap, m->cap, 1, d_species, d_energy, d_force, d_stress, nullptr,

@@ -458,11 +458,9 @@ gapgb_status build_sf_table(const HostModel &m, SFDev *t, std::string *err);
 void set_last_error(const std::string &s);
 
 // kernel launchers (nbr.cu, wacsf.cu, gpr.cu, reduce.cu)
-// lattice false: the structures' records of the last launch_prep still hold
-// (the same lattices and cutoff, an MD step between rebuilds)
 void launch_prep(const gapgb_model *m, Workspace &ws, int S, int N, const int *d_atom_off,
                  const int *d_species, const double *d_lat, const double *d_pos,
-                 double rcut, cudaStream_t st, bool allow_bins = false, bool lattice = true);
+                 double rcut, cudaStream_t st, bool allow_bins = false);
 // exact: the reference's bit-identical list (FP64 path, neighbour export);
 // otherwise the FP32 forms' cheaper geometry (same pairs up to last-bit
 // decisions at r = rcut, where every term vanishes)

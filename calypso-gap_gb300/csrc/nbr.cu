@@ -890,11 +890,10 @@ int grid_for_warps(int nwarps_needed) {
 
 void launch_prep(const gapgb_model *m, Workspace &ws, int S, int N, const int *d_atom_off,
                  const int *d_species, const double *d_lat, const double *d_pos, double rcut,
-                 cudaStream_t st, bool allow_bins, bool lattice) {
+                 cudaStream_t st, bool allow_bins) {
   constexpr int per = 128 / kPrepLanes;
-  if (lattice)
-    k_prep_struct<<<(S + per - 1) / per, 128, 0, st>>>(S, d_atom_off, d_lat, rcut,
-                                                       allow_bins ? 1 : 0, ws.sinfo, ws.d_flags);
+  k_prep_struct<<<(S + per - 1) / per, 128, 0, st>>>(S, d_atom_off, d_lat, rcut,
+                                                     allow_bins ? 1 : 0, ws.sinfo, ws.d_flags);
   k_prep_atoms<<<(N + 255) / 256, 256, 0, st>>>(N, S, d_atom_off, d_species, d_pos, m->d_sf,
                                                  ws.sinfo, ws.atom_struct, ws.apos, ws.frac32,
                                                  ws.pos2f, ws.d_flags);
