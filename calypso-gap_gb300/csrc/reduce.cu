@@ -92,51 +92,58 @@ __device__ __forceinline__ void write_struct(int s, int c, double v, int lgrad,
         lgrad ? -v * (1.0 / kGPa2eVPang) / sinfo[s].volume : 0.0;
 }
 
-// Per-structure sums of e_i and the virial in two fixed-order stages: block
-// (p, s) reduces part p of structure s's atoms (parts chosen from the batch
-// shape, so that a single large cell spreads over many SMs; FP64 adds are
-// slow on this part), then eight lanes per structure, one per sum, add its
-// parts in order.  512 atoms a part: four rounds of the block's loads (2048
-// atoms a part left the 32 768-atom MD cell on 16 SMs, 20 + 11 us a step
-// against 9 + 6).
+// Per-structure sums of e_i and the virial in two fixed-order stages: the parts
+// of a structure's atoms, then eight lanes per structure, one per sum, add its
+// parts in order.  A structure of up to 1023 atoms is one part, a larger one
+// na / 512 of them (four rounds of a block's loads; 2048 atoms a part left the
+// 32 768-atom MD cell on 16 SMs, 20 + 11 us a step against 9 + 6), whatever
+// the batch, so its sums are the same bit for bit alone and in any batch.
+// Blocks (x, s) share structure s's parts; how many there are follows the batch.
 constexpr int kMaxParts = 64;
+__host__ __device__ constexpr int parts_of(long na) {
+  return (int)(na < 1024 ? 1 : (na < 512 * kMaxParts ? na / 512 : kMaxParts));
+}
 
 __global__ void __launch_bounds__(128)
-    k_struct_partial(int parts, int lgrad, const StructInfo *__restrict__ sinfo,
+    k_struct_partial(int lgrad, const StructInfo *__restrict__ sinfo,
                      const double *__restrict__ e, const double *__restrict__ wvir,
                      double *__restrict__ atom_e, double *__restrict__ part) {
   __shared__ double red[7][128];
-  const int s = blockIdx.y, p = blockIdx.x;
+  const int s = blockIdx.y;
   const int a0 = sinfo[s].a0, na = sinfo[s].na;
-  const int len = (na + parts - 1) / parts;
-  const int beg = p * len, end = min(na, beg + len);
-  double acc[7] = {0, 0, 0, 0, 0, 0, 0};
+  const int parts = parts_of(na), len = (na + parts - 1) / parts;
   // upper triangle (a <= b) in the reference's k1 order: 11 12 13 22 23 33
   const int comp[6] = {0, 1, 2, 4, 5, 8};
-  for (int q = beg + threadIdx.x; q < end; q += blockDim.x) {
-    const int i = a0 + q;
-    acc[0] += e[i];
-    if (atom_e) atom_e[i] = e[i];
-    if (lgrad)
-      for (int c = 0; c < 6; ++c) acc[1 + c] += wvir[(size_t)i * 9 + comp[c]];
-  }
-  for (int c = 0; c < 7; ++c) red[c][threadIdx.x] = acc[c];
-  __syncthreads();
-  for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-    if (threadIdx.x < w)
-      for (int c = 0; c < 7; ++c) red[c][threadIdx.x] += red[c][threadIdx.x + w];
+  for (int p = blockIdx.x; p < parts; p += gridDim.x) {
+    const int beg = p * len, end = min(na, beg + len);
+    double acc[7] = {0, 0, 0, 0, 0, 0, 0};
+    for (int q = beg + threadIdx.x; q < end; q += blockDim.x) {
+      const int i = a0 + q;
+      acc[0] += e[i];
+      if (atom_e) atom_e[i] = e[i];
+      if (lgrad)
+        for (int c = 0; c < 6; ++c) acc[1 + c] += wvir[(size_t)i * 9 + comp[c]];
+    }
+    for (int c = 0; c < 7; ++c) red[c][threadIdx.x] = acc[c];
+    __syncthreads();
+    for (int w = blockDim.x / 2; w > 0; w >>= 1) {
+      if (threadIdx.x < w)
+        for (int c = 0; c < 7; ++c) red[c][threadIdx.x] += red[c][threadIdx.x + w];
+      __syncthreads();
+    }
+    if (threadIdx.x < 7) part[((size_t)s * kMaxParts + p) * 7 + threadIdx.x] = red[threadIdx.x][0];
     __syncthreads();
   }
-  if (threadIdx.x < 7) part[((size_t)s * parts + p) * 7 + threadIdx.x] = red[threadIdx.x][0];
 }
 
-__global__ void k_struct_final(int S, int parts, int lgrad, const StructInfo *__restrict__ sinfo,
+__global__ void k_struct_final(int S, int lgrad, const StructInfo *__restrict__ sinfo,
                                const double *__restrict__ part, double *__restrict__ energy,
                                double *__restrict__ stress) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x, s = t >> 3, c = t & 7;
   if (s >= S || c == 7) return;
+  const int parts = parts_of(sinfo[s].na);
   double v = 0.0;
-  for (int p = 0; p < parts; ++p) v += part[((size_t)s * parts + p) * 7 + c];
+  for (int p = 0; p < parts; ++p) v += part[((size_t)s * kMaxParts + p) * 7 + c];
   write_struct(s, c, v, lgrad, sinfo, energy, stress);
 }
 
@@ -157,13 +164,11 @@ void launch_forces(Workspace &ws, int N, int cap, double *d_force, cudaStream_t 
 
 void launch_struct_reduce(Workspace &ws, int S, int lgrad, double *d_energy, double *d_stress,
                           double *d_atom_e, int N, cudaStream_t st) {
-  // about 512 atoms per part for the mean structure size, at most kMaxParts
-  const long per = S > 0 ? (long)N / S : 0;
-  const int parts = (int)std::max(1L, std::min((long)kMaxParts, per / 512));
-  k_struct_partial<<<dim3(parts, S), 128, 0, st>>>(parts, lgrad, ws.sinfo, ws.e, ws.wvir, d_atom_e,
+  // as many blocks a structure as its mean size has parts
+  const int blocks = parts_of(S > 0 ? (long)N / S : 0);
+  k_struct_partial<<<dim3(blocks, S), 128, 0, st>>>(lgrad, ws.sinfo, ws.e, ws.wvir, d_atom_e,
                                                     ws.red_part);
-  k_struct_final<<<(S + 15) / 16, 128, 0, st>>>(S, parts, lgrad, ws.sinfo, ws.red_part, d_energy,
-                                                d_stress);
+  k_struct_final<<<(S + 15) / 16, 128, 0, st>>>(S, lgrad, ws.sinfo, ws.red_part, d_energy, d_stress);
 }
 
 template void launch_forces<double>(Workspace &, int, int, double *, cudaStream_t);
