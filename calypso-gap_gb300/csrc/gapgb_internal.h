@@ -225,17 +225,19 @@ struct W64Cut {
   int top;                     // biased exponent of 2^(E - 1)
   int up;                      // bits from the pairs' unit to the cutoff's own
   unsigned long long rc2;      // rc^2 in the pairs' unit
+  double rc2d;                 // rc^2
 };
 struct W64Fc {
   W64Cut c[kMaxRC];
   // fixed point: lengths below 2^(e - 1) in units of 2^(e - 64), their squares
   // in units of 2^(2 e - 64) (e: pairs), radial arguments in 2^(er - 64)
   int e, er;
+  int close;  // 1/(ab) whose high word is above this: the pair is formed in FP64
 };
 struct W64Exp {  // exp(a x) of an x in fixed point: see exp_neg
   double a;
   unsigned long long m;
-  int frac, pad;
+  int frac, steep;
 };
 // 2^(j/1024) in units of 2^-63 (gpr64_tc.cu)
 constexpr int kExpN = 1024;

@@ -126,13 +126,15 @@ __device__ __forceinline__ void fc_fix2(const W64Cut &c, u64 w, double &f, doubl
 // function in IEEE floating-point arithmetic", ACM TOMS 15, 1989) and
 // 2^(r/1024) by a degree-4 polynomial, all in integer arithmetic (exp2_fix of
 // gpr64_tc.cu).  The fraction is cut at 2^-50 (and 2^-50 off where it is zero):
-// a relative 2^-60.  Past the normal range, and for a > 0 (frac < 0), the
-// library's exp.
-__device__ __forceinline__ double exp_neg(const W64Exp &c, u64 x, int e,
-                                          const u64 *__restrict__ T) {
+// a relative 2^-60.  Past the normal range (|a v| >= 708), for a > 0 (frac < 0),
+// and where x is so small that its units are too coarse for the exponent
+// (c.steep and the caller's `small`), the value in FP64, f().
+template <typename F>
+__device__ __forceinline__ double exp_neg(const W64Exp &c, u64 x, const u64 *__restrict__ T,
+                                          bool small, F f) {
   const u64 hi = __umul64hi(x, c.m), lo = x * c.m;
   const u64 ki = hi >> (c.frac & 63);
-  if (c.frac < 0 || ki >= 1045929) return exp(c.a * fix_double(x >> 1, e - 63));  // |a v| >= 708
+  if (c.frac < 0 || (c.steep && small) || ki >= 1045929) return f();
   const u64 fr = c.frac >= 50 ? hi >> (c.frac - 50) : (hi << (50 - c.frac)) | (lo >> (14 + c.frac));
   const int k = -1 - (int)ki;
   const u64 t = T[k & (kExpN - 1)];
@@ -149,6 +151,13 @@ __device__ __forceinline__ double exp_neg(const W64Exp &c, u64 x, int e,
   const u64 m = t + (__umul64hi(t, p) >> 10);
   return __longlong_as_double(
       (i64)(((u64)(uint32_t)((k >> 10) + 1022) << 52) + (m >> 11) + ((m >> 10) & 1)));
+}
+
+// exp(a u2) of a slot's (r - rs)^2
+__device__ __forceinline__ double slot_exp(const W64Exp &c, double u2, const W64Fc &fc,
+                                           const u64 *__restrict__ T) {
+  const u64 x = to_fix(u2, fc.er - 1 + 1023);
+  return exp_neg(c, x, T, (x >> 53) == 0, [&] { return exp(c.a * u2); });
 }
 
 // sums v[0..N) over the warp's lanes by halving exchanges: at each step a
@@ -347,26 +356,60 @@ __device__ __forceinline__ unsigned upper(const View &s, int W, int j, int w) {
   return w > (j >> 5) ? m : (w < (j >> 5) ? 0u : m & ~((2u << (j & 31)) - 1u));
 }
 
-// A pair of slots in fixed point: c^2 and a^2 + b^2 + c^2 (units of 2^(2 e - 64)),
-// and (a^2 + b^2 - c^2) / 2.  The differences are below the cutoff, 2^(e - 1),
-// whatever wraps before.  Integer instructions, two FP64 ones less per
-// coordinate; the unit is finer than an FP64 square's last place from 0.1 A up.
+// A pair of slots: s3 = a^2 + b^2 + c^2 in units of 2^(2 e - 64), the argument of
+// fc(c), the cosine, and whether c is within the group's cutoff.  Formed in
+// fixed point: integer instructions, two FP64 ones less per coordinate.  The
+// differences are below the cutoff, 2^(e - 1), whatever wraps before; the dot
+// product is off by at most 2.5 of those units, so the cosine by less than
+// 2^-53 as long as a b is at least 2^(2 e - 9) (0.5 A^2 at a cutoff of 6 A, 8 at
+// 20).  Closer slots, and with them every pair within a cutoff far below the
+// longest, are formed in FP64 (fc.close: the high word of the largest 1/(ab)
+// that is not), and so are their steep exponentials.
 struct Pair {
-  u64 c2, s3;
-  i64 dot;
+  u64 s3, w;
+  double cosv;
+  bool in, close;
 };
-__device__ __forceinline__ Pair pair_of(const View &s, int j, int k) {
+__device__ __forceinline__ double pair_c2(const double4 &a, const double4 &b) {
+  const double x = a.x - b.x, y = a.y - b.y, z = a.z - b.z;
+  return fma(x, x, fma(y, y, z * z));
+}
+// exp(al s3), a factor per side (rare: a loop, so that it takes few registers)
+__device__ __forceinline__ double pair_exp(const double4 *A, int j, int k, double al) {
+  double e = 1.0;
+#pragma unroll 1
+  for (int u = 0; u < 3; ++u) {
+    const double r = A[u ? k : j].w;
+    e *= exp(al * (u < 2 ? r * r : pair_c2(A[j], A[k])));
+  }
+  return e;
+}
+__device__ __forceinline__ Pair pair_of(const View &s, int j, int k, double iab, const W64Fc &fc,
+                                        const W64Cut &cut) {
+  Pair p;
+  p.close = __double2hiint(iab) > fc.close;
+  if (p.close) {
+    const double4 a = s.A[j], b = s.A[k];
+    const double c2 = pair_c2(a, b);
+    p.s3 = to_fix(fma(a.w, a.w, fma(b.w, b.w, c2)), 2 * fc.e - 1 + 1023);
+    p.w = slot_arg(c2, cut);
+    p.in = c2 <= cut.rc2d;
+    p.cosv = fma(a.x, b.x, fma(a.y, b.y, a.z * b.z)) * iab;
+    return p;
+  }
   const I64x4 a = s.I[j], b = s.I[k];
   auto sq = [](i64 d) {
     const u64 m = (u64)(d < 0 ? -d : d);
     return __umul64hi(m, m);
   };
-  Pair p;
-  p.c2 = sq((i64)((u64)a.x - (u64)b.x)) + sq((i64)((u64)a.y - (u64)b.y)) +
-         sq((i64)((u64)a.z - (u64)b.z));
+  const u64 c2 = sq((i64)((u64)a.x - (u64)b.x)) + sq((i64)((u64)a.y - (u64)b.y)) +
+                 sq((i64)((u64)a.z - (u64)b.z));
   const u64 h = (u64)a.w + (u64)b.w;
-  p.s3 = 2 * h + p.c2;
-  p.dot = (i64)(h - (p.c2 >> 1));
+  p.s3 = 2 * h + c2;
+  p.w = pair_arg(c2, cut);
+  p.in = c2 <= cut.rc2;
+  // costheta = (rij^2 + rik^2 - rjk^2) / (2 rij rik) (wacsf.f90:271-273)
+  p.cosv = signed_double((i64)(h - (c2 >> 1)), 2 * fc.e - 64) * iab;
   return p;
 }
 
@@ -422,7 +465,7 @@ __global__ void __launch_bounds__(kBlk, NAL * (DEG + 1) <= 10 ? 5 : 3)
     double *Gi = G + (size_t)i * t.D;
     if (t.nrad > 0 && y == split - 1) {
       // radial terms: thread = (slot group, SF), so the lanes stay busy for
-      // any number of SFs; the slot groups are summed in order
+      // any number of SFs; the slot groups are summed in pairs
       const int ng = kBlk / t.nrad, sr = tid % t.nrad, gr = tid / t.nrad;
       double acc = 0.0, accw = 0.0;
       if (gr < ng) {
@@ -430,8 +473,8 @@ __global__ void __launch_bounds__(kBlk, NAL * (DEG + 1) <= 10 ? 5 : 3)
         const double rs = t.rad_rs[sr];
         const double2 *f = s.fc + (size_t)t.rad_rc[sr] * capS;
         for (int q = gr; q < P; q += ng) {
-          const double fq = f[q].x, u = s.A[q].w - rs;
-          const double e = exp_neg(ex, to_fix(u * u, fc.er - 1 + 1023), fc.er, s.T);
+          const double fq = f[q].x, u = s.A[q].w - rs, u2 = u * u;
+          const double e = slot_exp(ex, u2, fc, s.T);
           const double v = __double2hiint(fq) != 0 ? e * fq : 0.0;  // beyond the cutoff: zero
           acc += v;
           accw = fma(v, s.B[q].y, accw);
@@ -440,14 +483,18 @@ __global__ void __launch_bounds__(kBlk, NAL * (DEG + 1) <= 10 ? 5 : 3)
       rp[tid] = acc;
       rp[kBlk + tid] = accw;
       __syncthreads();
-      if (tid < t.nrad) {
-        double a = 0.0, w = 0.0;
-        for (int g = 0; g < ng; ++g) {
-          a += rp[g * t.nrad + tid];
-          w += rp[kBlk + g * t.nrad + tid];
+      for (int w = ng; w > 1;) {
+        const int h = (w + 1) / 2;
+        if (gr < w - h) {
+          rp[tid] += rp[tid + h * t.nrad];
+          rp[kBlk + tid] += rp[kBlk + tid + h * t.nrad];
         }
-        Gi[t.rad_d[tid]] = a;
-        Gi[t.rad_d[tid] + t.nsf] = w;
+        w = h;
+        __syncthreads();
+      }
+      if (tid < t.nrad) {
+        Gi[t.rad_d[tid]] = rp[tid];
+        Gi[t.rad_d[tid] + t.nsf] = rp[kBlk + tid];
       }
     }
     int u0 = 0;  // index of the group's first unit
@@ -473,13 +520,12 @@ __global__ void __launch_bounds__(kBlk, NAL * (DEG + 1) <= 10 ? 5 : 3)
           const bool live = p < p1;
           const unsigned jk = live ? s.list[p - p0] : 0u;
           const int j = jk & 0xffff, k = jk >> 16;
-          const Pair pr = pair_of(s, j, k);
           const double2 bj = s.B[j], bk = s.B[k];
-          double fcc = fc_fix(fc.c[rci], pair_arg(pr.c2, fc.c[rci]));
-          const bool in = live && pr.c2 <= fc.c[rci].rc2;  // else exactly zero
+          const Pair pr = pair_of(s, j, k, bj.x * bk.x, fc, fc.c[rci]);
+          double fcc = fc_fix(fc.c[rci], pr.w);
+          const bool in = live && pr.in;  // else exactly zero
           fcc = in ? fcc : 0.0;
-          // costheta = (rij^2 + rik^2 - rjk^2) / (2 rij rik) (wacsf.f90:271-273)
-          const double cosv = signed_double(pr.dot, 2 * fc.e - 64) * (bj.x * bk.x);
+          const double cosv = pr.cosv;
           const double F = f[j].x * f[k].x * fcc;
           const double wjk = bj.y * bk.y;
           const double uu = fma(0.5, cosv, 0.5), ww = fma(-0.5, cosv, 0.5);
@@ -501,7 +547,9 @@ __global__ void __launch_bounds__(kBlk, NAL * (DEG + 1) <= 10 ? 5 : 3)
           }
 #pragma unroll
           for (int q = 0; q < NAL; ++q) {
-            const double ef = in ? exp_neg(ex[q], pr.s3, 2 * fc.e, s.T) * F : 0.0;
+            const double ef = in ? exp_neg(ex[q], pr.s3, s.T, pr.close,
+                                           [&] { return pair_exp(s.A, j, k, ex[q].a); }) * F
+                                 : 0.0;
             const double efw = ef * wjk;
 #pragma unroll
             for (int n = 0; n < NB; ++n) {
@@ -704,7 +752,7 @@ __global__ void __launch_bounds__(kBlk, 4)
             u2 = u * u;
             ur = u * b.x;
           }
-          const double e = exp_neg(t.rad_e[a], to_fix(u2, fc.er - 1 + 1023), fc.er, s.T);
+          const double e = slot_exp(t.rad_e[a], u2, fc, s.T);
           const double g = fma(2.0 * al * ur, f.x, f.y);
           sum = fma(fma(dg[t.rad_d[a] + t.nsf], b.y, dg[t.rad_d[a]]) * e, g, sum);
         }
@@ -744,21 +792,23 @@ __global__ void __launch_bounds__(kBlk, 4)
           const bool live = p < p1;
           const unsigned jk = live ? s.list[p - p0] : 0u;
           const int j = jk & 0xffff, k = jk >> 16;
-          const Pair pr = pair_of(s, j, k);
           const double2 bj = s.B[j], bk = s.B[k], fj = f[j], fk = f[k];
+          const double iab = bj.x * bk.x;
+          const Pair pr = pair_of(s, j, k, iab, fc, fc.c[rci]);
           double fcc, fcd;
-          fc_fix2(fc.c[rci], pair_arg(pr.c2, fc.c[rci]), fcc, fcd);
+          fc_fix2(fc.c[rci], pr.w, fcc, fcd);
           fcd *= kd;
-          const bool in = live && pr.c2 <= fc.c[rci].rc2;
+          const bool in = live && pr.in;
           fcc = in ? fcc : 0.0;
           fcd = in ? fcd : 0.0;
-          const double iab = bj.x * bk.x;
-          const double cosv = signed_double(pr.dot, 2 * fc.e - 64) * iab;
+          const double cosv = pr.cosv;
           const double wjk = bj.y * bk.y;
           double SP = 0.0, SQ = 0.0, SU = 0.0;
 #pragma unroll
           for (int q = 0; q < NAL; ++q) {
-            const double e = in ? exp_neg(ex[q], pr.s3, 2 * fc.e, s.T) : 0.0;
+            const double e = in ? exp_neg(ex[q], pr.s3, s.T, pr.close,
+                                          [&] { return pair_exp(s.A, j, k, ex[q].a); })
+                                : 0.0;
             const double *U0 = sU + q * NB, *U1 = sU + (NAL + q) * NB;
             double pv = fma(wjk, U1[DEG], U0[DEG]), pd = 0.0;
 #pragma unroll
@@ -962,8 +1012,7 @@ __global__ void __launch_bounds__(kBlk)
       if ((__double2hiint(f.x) | __double2hiint(f.y)) == 0) continue;  // beyond the cutoff
       const double4 d = s.A[q];
       const double al = t.rad_e[a].a, u = d.w - t.rad_rs[a];
-      const double v = exp_neg(t.rad_e[a], to_fix(u * u, fc.er - 1 + 1023), fc.er, s.T) *
-                       fma(2.0 * al * (u * b.x), f.x, f.y);
+      const double v = slot_exp(t.rad_e[a], u * u, fc, s.T) * fma(2.0 * al * (u * b.x), f.x, f.y);
       const double dd[3] = {d.x, d.y, d.z};
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
@@ -988,19 +1037,21 @@ __global__ void __launch_bounds__(kBlk)
           if (p >= p1) continue;
           const unsigned jk = s.list[p - p0];
           const int j = jk & 0xffff, k = jk >> 16;
-          const Pair pr = pair_of(s, j, k);
           const double2 bj = s.B[j], bk = s.B[k], fj = f[j], fk = f[k];
+          const double iab = bj.x * bk.x;
+          const Pair pr = pair_of(s, j, k, iab, fc, fc.c[rci]);
           double fcc, fcd;
-          fc_fix2(fc.c[rci], pair_arg(pr.c2, fc.c[rci]), fcc, fcd);
-          const bool in = pr.c2 <= fc.c[rci].rc2;
+          fc_fix2(fc.c[rci], pr.w, fcc, fcd);
+          const bool in = pr.in;
           fcc = in ? fcc : 0.0;
           fcd = in ? fcd * kd : 0.0;
-          const double iab = bj.x * bk.x;
-          const double cosv = signed_double(pr.dot, 2 * fc.e - 64) * iab;
+          const double cosv = pr.cosv;
           double E[NAL];
 #pragma unroll
           for (int q = 0; q < NAL; ++q)
-            E[q] = in ? exp_neg(t.alpha[g][q], pr.s3, 2 * fc.e, s.T) : 0.0;
+            E[q] = in ? exp_neg(t.alpha[g][q], pr.s3, s.T, pr.close,
+                                [&] { return pair_exp(s.A, j, k, t.alpha[g][q].a); })
+                      : 0.0;
           const double fab = fj.x * fk.x, F = fab * fcc;
           const double ca = fma(-cosv, bj.x * bj.x, iab), cb = fma(-cosv, bk.x * bk.x, iab);
           const double ga = fcc * fk.x * fj.y, gb = fcc * fj.x * fk.y, gc = fab * fcd;
@@ -1111,9 +1162,13 @@ int split_of(int N) {
 
 namespace {
 
-// e = -alpha as exp_neg takes it, for arguments in units of 2^(E - 64)
-W64Exp exp_scale(double alpha, int E) {
-  W64Exp c = {-alpha, 0, 50, 0};
+// e = -alpha as exp_neg takes it, for arguments in units of 2^(E - 64) that are off
+// by up to `units` of them (a pair's s3: 4, a slot's (r - rs)^2: 1).  Steep: that
+// passes 2^-52 of the exponent (pairs from alpha = 4 at a cutoff of 6 A, slots
+// from 64), so only arguments large enough for FP64 products to be off by as
+// much take the units.
+W64Exp exp_scale(double alpha, int E, int units) {
+  W64Exp c = {-alpha, 0, 50, std::ldexp(std::fabs(alpha) * units, E) > 4096.0};
   if (alpha == 0.0) return c;
   const DD v = dd_mul({alpha, 0.0}, {0x1.71547652b82fep+10, 0x1.777d0ffda0d24p-46});
   int ea;
@@ -1149,6 +1204,7 @@ bool w64_table(const SFDev &s, W64Tab *t) {
   }
   std::frexp(1.001 * rmax, &t->fc.e);
   t->fc.e += 1;
+  t->fc.close = (1023 + 9 - 2 * t->fc.e) * (1 << 20) - 1;
   std::frexp(std::max(u2max, 1e-30) * 1.001, &t->fc.er);
   for (int q = 0; q < s.nrc; ++q) {
     t->rc[q] = s.rc_val[q];
@@ -1157,12 +1213,13 @@ bool w64_table(const SFDev &s, W64Tab *t) {
     t->fc.c[q].up = 2 * t->fc.e - (t->fc.c[q].top - 1022);
     if (t->fc.c[q].up > 62) return false;
     t->fc.c[q].rc2 = (unsigned long long)std::ldexp(s.rc_val[q] * s.rc_val[q], 64 - 2 * t->fc.e);
+    t->fc.c[q].rc2d = s.rc_val[q] * s.rc_val[q];
     t->kd[q] = -t->kv[q];  // fc'(r) / r = (d fc / dw) kv
   }
   for (int q = 0; q < s.nrad; ++q) {
     t->rad_d[q] = s.rad_d[q];
     t->rad_rc[q] = s.rad_rc[q];
-    t->rad_e[q] = exp_scale(s.rad_alpha[q], t->fc.er);
+    t->rad_e[q] = exp_scale(s.rad_alpha[q], t->fc.er, 1);
     t->rad_rs[q] = s.rad_rs[q];
   }
   int nal = 1, deg = 1;
@@ -1179,7 +1236,7 @@ bool w64_table(const SFDev &s, W64Tab *t) {
       while (q < n && t->alpha[g][q].a != -al) ++q;
       if (q == 4) return false;
       if (q == n) {
-        t->alpha[g][n++] = exp_scale(al, 2 * t->fc.e);
+        t->alpha[g][n++] = exp_scale(al, 2 * t->fc.e, 4);
       }
       t->ang_d[a] = s.ang_d[a];
       t->ang_g[a] = g;
