@@ -26,7 +26,7 @@
 // forward substitution, its trailing updates beside the next block's factor
 // and panel, and a back substitution of one launch per block.  No kernel
 // waits on another CTA.  Measured per call: 48 alloy512 cells and 1500 points
-// 45.5 -> 10.2 ms, 8 Si cells of 64 atoms with forces and stresses and 150
+// 45.5 -> 8.4 ms, 8 Si cells of 64 atoms with forces and stresses and 150
 // points 91 -> 3.2 ms.
 #include <algorithm>
 #include <string>

@@ -227,7 +227,7 @@ struct W64Cut {
   unsigned long long rc2;      // rc^2 in the pairs' unit
   double rc2d;                 // rc^2
 };
-struct W64Fc {
+struct W64Fc {  // passed by value, for the constant bank
   W64Cut c[kMaxRC];
   // fixed point: lengths below 2^(e - 1) in units of 2^(e - 64), their squares
   // in units of 2^(2 e - 64) (e: pairs), radial arguments in 2^(er - 64)
@@ -244,7 +244,7 @@ constexpr int kExpN = 1024;
 const unsigned long long *exp2_table();
 struct W64Tab {
   int nsf, D, nrad, nang, nrc, ngrp, nal, deg;  // nal, deg: the kernels' template sizes
-  double rc[kMaxRC], kv[kMaxRC], kd[kMaxRC];
+  double rc[kMaxRC], kd[kMaxRC];
   int rad_d[kMaxSF], rad_rc[kMaxSF];
   W64Exp rad_e[kMaxSF];  // a = -alpha
   double rad_rs[kMaxSF];
@@ -252,7 +252,6 @@ struct W64Tab {
   W64Exp alpha[kMaxRC][4];
   int ang_d[kMaxSF], ang_g[kMaxSF], ang_q[kMaxSF];
   double bern[kMaxSF][5], mono[kMaxSF][5];
-  W64Fc fc;  // the cutoffs' polynomials (also passed by value, for the constant bank)
 };
 
 struct StructInfo {
@@ -368,6 +367,7 @@ struct gapgb_model {
   gapgb::SFT<float> *d_sft32 = nullptr;
   gapgb::SFT<float> sft32h{};          // host copy (kernel selection)
   gapgb::W64Tab w64h{};                // FP64 descriptor kernels' table (wacsf64.cu)
+  gapgb::W64Fc w64fc{};                // and the cutoffs' polynomials
   gapgb::W64Tab *d_w64 = nullptr;
   unsigned long long *d_exp64 = nullptr;  // exp2_table
   bool w64_tried = false;              // w64_prepare ran (d_w64 stays null: the set does not qualify)

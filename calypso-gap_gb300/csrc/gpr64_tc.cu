@@ -170,7 +170,7 @@ __global__ void __launch_bounds__(256)
 // digits and norm: 16 lanes per row (8 components each).  Shared by atoms
 // and sparse points.  Returns the norm |x|^2/2 in units of 2^-52 modulo 2^64
 // on every lane; bf is it in FP32; e the exponent, |x| < 2^e.
-__device__ __forceinline__ i64 row_digits(const double (&x)[8], int lane16, int &e, float &bf,
+__device__ __forceinline__ i64 row_digits(const double (&x)[8], int &e, float &bf,
                                           i64 (&X)[8], bool &nan) {
   int me = -1022;
   bool bad = false;
@@ -206,7 +206,6 @@ __device__ __forceinline__ i64 row_digits(const double (&x)[8], int lane16, int 
   const i64 n = (i64)(u64)((q2 + ((unsigned __int128)1 << (sh - 1))) >> sh);
   const double top = (double)(u64)(q2 >> 64) * 18446744073709551616.0 + (double)(u64)q2;
   bf = (float)ldexp(top, 2 * e - 121);
-  (void)lane16;
   return n;
 }
 
@@ -232,7 +231,7 @@ __global__ void __launch_bounds__(128)
   float bf;
   i64 X[8];
   bool nan;
-  const i64 n = row_digits(x, lane16, e, bf, X, nan);
+  const i64 n = row_digits(x, e, bf, X, nan);
   unsigned char *tile = img + (size_t)(i / kR) * kS1 * slice1(KD);
   if (lane16 * 8 < KD)
     store_digits<kS1>(X, tile + kmajor_off(i % kR, lane16 * 8, KD / 8), slice1(KD));
@@ -268,7 +267,7 @@ __global__ void __launch_bounds__(128)
   float bf;
   i64 X[8];
   bool nan;
-  const i64 n = row_digits(x, lane16, e, bf, X, nan);
+  const i64 n = row_digits(x, e, bf, X, nan);
   if (k >= Mp) return;
   unsigned char *tile = img + (size_t)(k / kT1) * tile1(KD);
   if (lane16 * 8 < KD)

@@ -29,14 +29,13 @@
 // so fewer, wider MMAs, and W in tensor memory: 760 + 500 cycles a tile.
 // Two warps issue because a warp's next barrier poll waits for the MMAs that it
 // has queued: with one, the pipe idles 350 cycles after each batch of eight.
-// Measured: a tile (128 atoms x 64 points) takes about 1650 cycles, 19 us x
-// M / 1000 for up to 152 x 128 atoms, 43 to 47 % of the tensor pipe's cycles
-// and 57 to 62 % of the issue slots; 19456 atoms, M = 4000: 61 us, where a
-// kernel of 4 warps per 128 atoms and two CTAs per SM, each with its GEMMs and
-// epilogue in turn and A and W in shared memory, took 131; 16384 atoms,
-// M = 8000: 108 us (241).  The [mh; ml] and [mhT; mlT] pairs are adjacent 64-row
-// blocks in shared memory, which is the 128-row B operand of the same canonical
-// layout.
+// Measured: a tile (128 atoms x 64 points) takes about 1650 cycles, 43 to 47 %
+// of the tensor pipe's cycles and 57 to 62 % of the issue slots; a wave of up to
+// 152 x 128 atoms takes 61 us at M = 4000 and 108 at M = 8000, where a kernel of
+// 4 warps per 128 atoms and two CTAs per SM, each with its GEMMs and epilogue in
+// turn and A and W in shared memory, took 131 and 241.  The [mh; ml] and
+// [mhT; mlT] pairs are adjacent 64-row blocks in shared memory, which is the
+// 128-row B operand of the same canonical layout.
 //
 // Operand tiles use the no-swizzle K-major canonical layout: 8-row x 16-byte
 // core matrices, K-adjacent cores 128 B apart (LBO), 8-row groups

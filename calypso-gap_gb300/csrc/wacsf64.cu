@@ -18,7 +18,8 @@
 //    and the exponential (a 1024-entry table of 2^(j/1024) and a degree-4
 //    polynomial, argument reduction included) run in 64-bit fixed point on the
 //    integer pipe, where an instruction costs an SM sub-partition 1 to 2
-//    cycles, not 64; errors below 0.5 and 1 ulp;
+//    cycles, not 64; errors of the two functions below 0.5 and 1 ulp, pairs too
+//    close for the units in FP64 (pair_of);
 //  - the (1 +- cos)^zeta of a cutoff group are combinations of the products
 //    u^n w^(DEG-n) (u = (1 + cos)/2, w = 1 - u) with non-negative weights: a
 //    pair adds those products, times each alpha's exponential, to moments;
@@ -42,7 +43,8 @@
 // (unit mod 8) in order, and classes in order; a slot's gradient is summed
 // over its pairs in order after the pairs' scalars are written, by the same
 // block (split = 1) or by a second kernel.  Nothing is atomic, so results are
-// the same bit for bit in every run and in every batch.
+// the same bit for bit in every run and in every batch (short of one whose scratch
+// cannot be allocated, which takes wacsf.cu's kernels).
 #include <algorithm>
 #include <cmath>
 #include <vector>
@@ -851,7 +853,7 @@ __global__ void __launch_bounds__(kBlk, 4)
 // k_w64_finish, which adds them in order.
 constexpr int kGatherThreads = 512;
 __global__ void __launch_bounds__(kGatherThreads)
-    k_w64_gather(int N, int cap, int capS, const int *__restrict__ cnt,
+    k_w64_gather(int cap, int capS, const int *__restrict__ cnt,
                  const double4 *__restrict__ xyzr, const int *__restrict__ nj,
                  const double4 *__restrict__ apos, const float4 *__restrict__ d32,
                  const W64Tab *__restrict__ tab, const __grid_constant__ W64Fc fc,
@@ -935,15 +937,15 @@ DD dd_div(DD a, double b) {
 // stays at most 1): the power series of cos(sqrt(t)), t = (2 k^2 / kv) w,
 // in powers of v = 2 w - 1 to degree 18, economised to degree 11 by Chebyshev
 // polynomials (largest error 2e-17, the derivative's 5e-17), then in powers of
-// w, whose signs alternate.  Coefficients in units of 2^-61.
-void fc_series(double rc, double *kv, W64Cut *cut) {
+// w, whose signs alternate.  Coefficients in units of 2^-61.  Returns kv.
+double fc_series(double rc, W64Cut *cut) {
   const double k = kPiRef / rc;
   const double k2 = 2.0 / (rc * rc);
   float kf = (float)k2;
   if ((double)kf > k2) kf = std::nextafter(kf, 0.f);
-  *kv = (double)kf;
+  const double kv = (double)kf;
   constexpr int kDeg = 18, kTerms = 28;
-  const DD w = dd_div(dd_mul({k, 0.0}, {k, 0.0}), *kv);
+  const DD w = dd_div(dd_mul({k, 0.0}, {k, 0.0}), kv);
   DD a[kDeg + 1] = {};
   DD u = {0.5, 0.0};  // (-w)^n / (2 (2n)!)
   double row[kTerms + 1] = {1.0};  // C(n, m)
@@ -975,9 +977,10 @@ void fc_series(double rc, double *kv, W64Cut *cut) {
   }
   // 2^(E - 1) < rc^2 <= 2^E; kv / 2 in units of 2^(-63 - E)
   int E;
-  if (std::frexp(2.0 / *kv, &E) == 0.5) --E;  // rc^2 a power of two
+  if (std::frexp(2.0 / kv, &E) == 0.5) --E;  // rc^2 a power of two
   cut->top = E - 1 + 1023;
-  cut->ratio = (unsigned long long)std::ldexp(*kv * 0.5, E + 63);
+  cut->ratio = (unsigned long long)std::ldexp(kv * 0.5, E + 63);
+  return kv;
 }
 
 // The Jacobian J[i][slot][xyz][d] = dG_id / dp_slot of atoms [0, N): what the
@@ -1186,8 +1189,9 @@ W64Exp exp_scale(double alpha, int E, int units) {
 }
 
 // The table of a model, or false when its SF set keeps the generic kernels.
-bool w64_table(const SFDev &s, W64Tab *t) {
+bool w64_table(const SFDev &s, W64Tab *t, W64Fc *fc) {
   *t = W64Tab{};
+  *fc = W64Fc{};
   t->nsf = s.nsf;
   t->D = s.D;
   t->nrad = s.nrad;
@@ -1202,24 +1206,24 @@ bool w64_table(const SFDev &s, W64Tab *t) {
     const double u = std::max(std::fabs(s.rad_rs[q]), std::fabs(s.rc_val[s.rad_rc[q]] - s.rad_rs[q]));
     u2max = std::max(u2max, u * u);
   }
-  std::frexp(1.001 * rmax, &t->fc.e);
-  t->fc.e += 1;
-  t->fc.close = (1023 + 9 - 2 * t->fc.e) * (1 << 20) - 1;
-  std::frexp(std::max(u2max, 1e-30) * 1.001, &t->fc.er);
+  std::frexp(1.001 * rmax, &fc->e);
+  fc->e += 1;
+  fc->close = (1023 + 9 - 2 * fc->e) * (1 << 20) - 1;
+  std::frexp(std::max(u2max, 1e-30) * 1.001, &fc->er);
   for (int q = 0; q < s.nrc; ++q) {
     t->rc[q] = s.rc_val[q];
-    fc_series(s.rc_val[q], &t->kv[q], &t->fc.c[q]);
+    const double kv = fc_series(s.rc_val[q], &fc->c[q]);
     // (a cutoff 2^30 times shorter than the longest: left to the generic kernels)
-    t->fc.c[q].up = 2 * t->fc.e - (t->fc.c[q].top - 1022);
-    if (t->fc.c[q].up > 62) return false;
-    t->fc.c[q].rc2 = (unsigned long long)std::ldexp(s.rc_val[q] * s.rc_val[q], 64 - 2 * t->fc.e);
-    t->fc.c[q].rc2d = s.rc_val[q] * s.rc_val[q];
-    t->kd[q] = -t->kv[q];  // fc'(r) / r = (d fc / dw) kv
+    fc->c[q].up = 2 * fc->e - (fc->c[q].top - 1022);
+    if (fc->c[q].up > 62) return false;
+    fc->c[q].rc2 = (unsigned long long)std::ldexp(s.rc_val[q] * s.rc_val[q], 64 - 2 * fc->e);
+    fc->c[q].rc2d = s.rc_val[q] * s.rc_val[q];
+    t->kd[q] = -kv;  // fc'(r) / r = (d fc / dw) kv
   }
   for (int q = 0; q < s.nrad; ++q) {
     t->rad_d[q] = s.rad_d[q];
     t->rad_rc[q] = s.rad_rc[q];
-    t->rad_e[q] = exp_scale(s.rad_alpha[q], t->fc.er, 1);
+    t->rad_e[q] = exp_scale(s.rad_alpha[q], fc->er, 1);
     t->rad_rs[q] = s.rad_rs[q];
   }
   int nal = 1, deg = 1;
@@ -1236,7 +1240,7 @@ bool w64_table(const SFDev &s, W64Tab *t) {
       while (q < n && t->alpha[g][q].a != -al) ++q;
       if (q == 4) return false;
       if (q == n) {
-        t->alpha[g][n++] = exp_scale(al, 2 * t->fc.e, 4);
+        t->alpha[g][n++] = exp_scale(al, 2 * fc->e, 4);
       }
       t->ang_d[a] = s.ang_d[a];
       t->ang_g[a] = g;
@@ -1266,7 +1270,7 @@ bool w64_table(const SFDev &s, W64Tab *t) {
 gapgb_status w64_prepare(gapgb_model *m) {
   if (m->d_w64 || m->w64_tried) return GAPGB_OK;
   m->w64_tried = true;
-  if (!w64_table(m->sfh, &m->w64h)) return GAPGB_OK;
+  if (!w64_table(m->sfh, &m->w64h, &m->w64fc)) return GAPGB_OK;
   GAPGB_CUDA_TRY(cudaMalloc(&m->d_exp64, 8 * kExpN));
   GAPGB_CUDA_TRY(cudaMemcpy(m->d_exp64, exp2_table(), 8 * kExpN, cudaMemcpyHostToDevice));
   GAPGB_CUDA_TRY(cudaMalloc(&m->d_w64, sizeof(W64Tab)));
@@ -1357,7 +1361,7 @@ void launch_w64_fwd(const gapgb_model *m, Workspace &ws, int N, int cap, int cap
   if (fwd_bytes(t, N) > std::min(kScratchMax, ws.w64_bytes)) split = 1;
   const int gx = std::min(N, 1 << 20);
   f<<<dim3(gx, split), kBlk, smem, st>>>(N, cap, capS, ws.nbr_cnt, ws.nbr_xyz, ws.nbr_j, ws.apos,
-                                         ws.nbr_d32, m->d_w64, m->w64h.fc, m->d_exp64,
+                                         ws.nbr_d32, m->d_w64, m->w64fc, m->d_exp64,
                                          (double *)ws.G, (double *)ws.w64_scratch, split);
   if (split > 1 && t.nang > 0)
     k_w64_final<<<N, kBlk, 0, st>>>(N, NB, NM, m->d_w64, (const double *)ws.w64_scratch,
@@ -1384,7 +1388,7 @@ void launch_w64_bwd(const gapgb_model *m, Workspace &ws, int N, int cap, int cap
   int *first = (int *)(rad + (split > 1 ? (size_t)N * capS : 0));
   if (t.ngrp <= 1) gp = nullptr;
   b<<<dim3(gx, split), kBlk, smem, st>>>(N, cap, capS, ws.nbr_cnt, ws.nbr_xyz, ws.nbr_j, ws.apos,
-                                         ws.nbr_d32, m->d_w64, m->w64h.fc, m->d_exp64,
+                                         ws.nbr_d32, m->d_w64, m->w64fc, m->d_exp64,
                                          (const double *)ws.dedg, (double4 *)ws.gslot, ws.wvir, sc,
                                          rad, first, nsc, split);
   if (split > 1) {
@@ -1394,12 +1398,12 @@ void launch_w64_bwd(const gapgb_model *m, Workspace &ws, int N, int cap, int cap
     // 31 us at 128 threads, 43 at 512)
     const int th = std::min(kGatherThreads, std::max(kBlk, (2 * capS + 63) / 64 * 64));
     k_w64_gather<<<dim3(N, std::max(1, t.ngrp)), th, sg, st>>>(
-        N, cap, capS, ws.nbr_cnt, ws.nbr_xyz, ws.nbr_j, ws.apos, ws.nbr_d32, m->d_w64, m->w64h.fc,
+        cap, capS, ws.nbr_cnt, ws.nbr_xyz, ws.nbr_j, ws.apos, ws.nbr_d32, m->d_w64, m->w64fc,
         (double4 *)ws.gslot, ws.wvir, sc, rad, first, gp, nsc);
     if (gp) {
       kernel_smem((const void *)k_w64_finish, (int)sg, true);
       k_w64_finish<<<N, kBlk, sg, st>>>(cap, capS, ws.nbr_cnt, ws.nbr_xyz, ws.nbr_j, ws.apos,
-                                        ws.nbr_d32, m->d_w64, m->w64h.fc, (double4 *)ws.gslot,
+                                        ws.nbr_d32, m->d_w64, m->w64fc, (double4 *)ws.gslot,
                                         ws.wvir, rad, gp);
     }
   }
@@ -1421,7 +1425,7 @@ bool launch_w64_jac(const gapgb_model *m, Workspace &ws, int N, int cap, int cap
   if (!grow_scratch(ws, &ws.w64_scratch, &ws.w64_bytes, gx * nsc * 32, gx * nsc * 32, st))
     return false;
   f<<<gx, kBlk, smem, st>>>(N, cap, capS, ws.nbr_cnt, ws.nbr_xyz, ws.nbr_j, ws.apos, ws.nbr_d32,
-                            m->d_w64, t.fc, m->d_exp64, J, (double4 *)ws.w64_scratch, nsc, na);
+                            m->d_w64, m->w64fc, m->d_exp64, J, (double4 *)ws.w64_scratch, nsc, na);
   return true;
 }
 
