@@ -532,6 +532,12 @@ def roofline(stages, N, D, precision, simt=None, plain_stages=None, P=P_SLOTS, T
             ach = fl / (st * 1e-3) / 1e12
             pl[name] = {"achieved_tflops": ach,
                         "frac": ach / fp64_peak if fp64_peak else None}
+        # the GPR's contractions run on the tensor cores, as 36 BF16 products of
+        # base-256 digits each: its fraction of the FP64 FMA rate says how far past
+        # it they are, this one what the tensor cores give
+        digits = 36.0 * pl["gpr"]["achieved_tflops"]
+        pl["gpr"].update(digit_tflops=digits, digit_frac=digits / peaks["bf16_tflops"],
+                         digit_peak_source=src + " bf16_tflops")
         roof["plain_fp64"] = pl
     return roof
 
