@@ -709,17 +709,19 @@ __global__ void __launch_bounds__(kR)
 
 // phi[s][k] += sum over the structures' atoms within [i0, i1) of K_ik (W: the
 // kernel values of the row tiles from i0 on); the first part of a structure
-// sets.  A warp per (structure, point), lanes over rows: fixed order.
+// sets.  A warp per (structure, point), lanes over rows: fixed order.  An atom
+// whose descriptors are not numbers (its W is zero) makes the sum NaN.
 __global__ void __launch_bounds__(256)
     k_g64_phi(int i0, int i1, int Mp, int Mf, const int *__restrict__ off,
-              const double *__restrict__ W, double *__restrict__ phi) {
+              const int *__restrict__ rowexp, const double *__restrict__ W,
+              double *__restrict__ phi) {
   const int s = blockIdx.y, lane = threadIdx.x & 31;
   const int k = blockIdx.x * 8 + (threadIdx.x >> 5);
   const int a0 = max(off[s], i0), a1 = min(off[s + 1], i1);
   if (k >= Mf || (a0 >= a1 && off[s] != off[s + 1])) return;
   double v = 0.0;
   for (int i = a0 + lane; i < a1; i += 32)
-    v += W[((size_t)((i - i0) / kR) * Mp + k) * kR + (i - i0) % kR];
+    v += rowexp[i] == kRowNaN ? nan("") : W[((size_t)((i - i0) / kR) * Mp + k) * kR + (i - i0) % kR];
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   if (lane == 0) {
@@ -929,7 +931,7 @@ bool launch_gpr64(const gapgb_model *m, Workspace &ws, int N, cudaStream_t st) {
 }
 
 // Kernel values without coefficients, for the fit: row tiles in chunks.
-// use(first row, row tiles, W) enqueues what reads them.
+// use(first row, row tiles, every row's rowexp, W) enqueues what reads them.
 template <typename F>
 static bool g64_kernel_values(const gapgb_model *m, Workspace &ws, int N, const double *X,
                               cudaStream_t st, F use) {
@@ -952,7 +954,7 @@ static bool g64_kernel_values(const gapgb_model *m, Workspace &ws, int N, const 
         g.nt1, g.Mp, q + r.img + (size_t)c0 * kS1 * slice1(g.KD), row + (size_t)c0 * kR,
         p + g.img1, (const Col *)(p + g.col), (const u64 *)(p + g.tab), (double *)(q + r.W),
         nullptr, ws.d_flags);
-    use(c0 * kR, ct, (const double *)(q + r.W));
+    use(c0 * kR, ct, (const int *)(q + r.rowexp), (const double *)(q + r.W));
   }
   return true;
 }
@@ -961,9 +963,9 @@ static bool g64_kernel_values(const gapgb_model *m, Workspace &ws, int N, const 
 bool launch_phi64(const gapgb_model *m, Workspace &ws, int N, int S, int Mf, const int *d_off,
                   const double *G, double *phi, cudaStream_t st) {
   const int Mp = g64_layout(m->host.M, m->host.D).Mp;
-  return g64_kernel_values(m, ws, N, G, st, [&](int i0, int ct, const double *W) {
+  return g64_kernel_values(m, ws, N, G, st, [&](int i0, int ct, const int *rowexp, const double *W) {
     k_g64_phi<<<dim3((Mf + 7) / 8, S), 256, 0, st>>>(i0, std::min(N, i0 + ct * kR), Mp, Mf, d_off,
-                                                     W, phi);
+                                                     rowexp, W, phi);
   });
 }
 
@@ -973,7 +975,7 @@ bool launch_kmm64(const gapgb_model *m, Workspace &ws, int Mf, double *A, cudaSt
   const G64 g = g64_layout(M, m->host.D);
   if (!m->d_g64) return false;
   return g64_kernel_values(m, ws, M, (const double *)(m->d_g64 + g.mm), st,
-                           [&](int i0, int ct, const double *W) {
+                           [&](int i0, int ct, const int *, const double *W) {
                              k_g64_kmm<<<dim3((Mf + 31) / 32, ct * (kR / 32)), 256, 0, st>>>(
                                  M, i0, g.Mp, Mf, W, A);
                            });
