@@ -372,14 +372,21 @@ __device__ __forceinline__ void image_box(const float ext[3], const int nabc[3],
 
 // FP32 screen of an image: squared Cartesian length of (f_j - f_i + n) L.
 // Candidates farther than rcut + margin cannot pass the exact test (the
-// margin covers the FP32 rounding of the fractional coordinates).
+// margin covers the FP32 rounding of the fractional coordinates).  Every
+// operation's rounding is spelled out: the general loops of k_nbr_build count
+// the survivors in one place and queue them in another, and with the
+// contraction left to the compiler the two disagreed in the last bit, so that a
+// candidate exactly on the bound was counted but not queued, and whatever the
+// queue held there was taken for a neighbour.
 __device__ __forceinline__ float screen_r2(const float *L32, const float fd[3], int n1, int n2,
                                            int n3) {
-  const float a = fd[0] + (float)n1, b = fd[1] + (float)n2, c = fd[2] + (float)n3;
-  const float x = a * L32[0] + b * L32[3] + c * L32[6];
-  const float y = a * L32[1] + b * L32[4] + c * L32[7];
-  const float z = a * L32[2] + b * L32[5] + c * L32[8];
-  return x * x + y * y + z * z;
+  const float a = __fadd_rn(fd[0], (float)n1), b = __fadd_rn(fd[1], (float)n2),
+              c = __fadd_rn(fd[2], (float)n3);
+  float v[3];
+#pragma unroll
+  for (int k = 0; k < 3; ++k)
+    v[k] = __fmaf_rn(c, L32[6 + k], __fmaf_rn(b, L32[3 + k], __fmul_rn(a, L32[k])));
+  return __fmaf_rn(v[2], v[2], __fmaf_rn(v[1], v[1], __fmul_rn(v[0], v[0])));
 }
 
 constexpr int kQueue = 256;  // survivors per warp per exact-test round
