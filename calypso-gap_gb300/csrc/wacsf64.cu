@@ -294,7 +294,8 @@ __device__ __forceinline__ int stage(const View &s, const W64Tab &t, const W64Fc
 // of 4e-5 on the squared lengths (the FP32 records are off by less than 1e-6
 // of rc^2): pairs just outside the cutoff may be listed, and contribute
 // exactly zero.  The screen's arithmetic is even in (j, k), so bits (j, k) and
-// (k, j) agree.  Ends with a barrier.
+// (k, j) agree, and its rounding is spelled out, so the lists of k_w64_bwd and
+// k_w64_gather do (a pair's scalars are found by its place).  Ends with a barrier.
 template <bool FULL>
 __device__ __forceinline__ int build_pairs(const View &s, const W64Tab &t, int g, int P, int &n) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
@@ -321,7 +322,7 @@ __device__ __forceinline__ int build_pairs(const View &s, const W64Tab &t, int g
       bool in = k < n && (FULL ? k != j : k > j);
       const float4 ak = s.f4[s.idx[in ? k : j]];
       const float cx = aj.x - ak.x, cy = aj.y - ak.y, cz = aj.z - ak.z;
-      in = in && cx * cx + cy * cy + cz * cz <= c2m;
+      in = in && __fmaf_rn(cz, cz, __fmaf_rn(cy, cy, __fmul_rn(cx, cx))) <= c2m;
       const unsigned m = __ballot_sync(0xffffffffu, in);
       if (lane == 0) {
         s.mask[j * W + w] = m;
