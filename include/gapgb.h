@@ -428,7 +428,9 @@ gapgb_status gapgb_gpr_labels(gapgb_model *model, int nstruct,
  * Each step is one CUDA graph launch.  gapgb_md_create evaluates the forces
  * at t = 0 (growing the neighbour capacity with 25 % headroom) and captures
  * the two step graphs; the model is dedicated to the MD object while it
- * lives (its workspace holds the list) and must not be reconfigured. */
+ * lives (its workspace holds the list) and must not be reconfigured.  Every
+ * step reads d_lat: a caller may strain cells and positions between runs (the
+ * strain counts towards the atoms' displacement). */
 typedef struct gapgb_md gapgb_md;
 gapgb_status gapgb_md_create(gapgb_model *model, int nstruct, int natoms,
                              const int *d_atom_off, const int *d_species,
